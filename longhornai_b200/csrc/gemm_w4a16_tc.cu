@@ -373,7 +373,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     int* final_tile = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 3));   // column tile this CTA sums at its end, or -1
     float* inv_s = reinterpret_cast<float*>(tmem_slot + 4);          // [MP]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto raw_full = [&](int s) { return bar0 + 8 * s; };
     auto raw_empty = [&](int s) { return bar0 + 8 * (RS + s); };
@@ -470,8 +470,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: per unit, two 128-column tiles x eight k16 steps ----
-        if (lane == 0) {
+        // ---- MMA issuer: per unit, two 128-column tiles x four k32 steps ----
+        if (ptx::elect_one()) {
             for (int i = 0; i < n_units; ++i) {
                 const int bs = i % BS;
                 if (!ptx::mbar_wait(b_full(bs), (i / BS) & 1, abort_flag, p.status)) break;

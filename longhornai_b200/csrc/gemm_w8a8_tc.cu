@@ -237,7 +237,7 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8 * s; };
     auto empty_bar = [&](int s) { return bar0 + 8 * (W8_STAGES + s); };
@@ -292,7 +292,7 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             int it = 0, ti = 0;
             for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x, ++ti) {
                 const int buf = ti & 1;
@@ -399,7 +399,7 @@ gemm_w8a8_tc_pair_kernel(const __grid_constant__ TensorMap tmA, const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_ctarank();       // 0 = leader
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8 * s; };
@@ -449,7 +449,7 @@ gemm_w8a8_tc_pair_kernel(const __grid_constant__ TensorMap tmA, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && ptx::elect_one()) {
             int it = 0, ti = 0;
             for (int tile = pair; tile < n_tiles && !*abort_flag; tile += n_pairs, ++ti) {
                 const int buf = ti & 1;
