@@ -233,6 +233,19 @@ static int check_attn(const lhb_paged_attn_cfg* cfg, const lhb_paged_layout* L) 
     return LHB_OK;
 }
 
+// One query row per request: split-KV decode kernel.  Several rows, other head dims, page sizes or
+// unaligned pointers: the generic kernel.
+static int dispatch_attn_q8(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp, const float* Ks,
+                            const float* Vs, const int32_t* tables, int max_blocks, const int32_t* seq_lens, int seq_len,
+                            int n_req, float* O, const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L, cudaStream_t st) {
+    if (aligned16(Q) && aligned16(Kp) && aligned16(Vp) && aligned16(Ks) && aligned16(Vs) && aligned16(O)) {
+        if (decode_fast_ok(cfg, L))
+            return launch_decode_fast(ctx, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, seq_len, n_req, O, cfg, L, st);
+    }
+    return launch_paged_attention_generic(ctx, true, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, seq_len, n_req, O,
+                                          cfg, L, st);
+}
+
 int lhb_paged_attention_q8_batched(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp,
                                    const float* Ks, const float* Vs, const int32_t* tables,
                                    int max_blocks, const int32_t* seq_lens, int n_req, float* O,
@@ -243,14 +256,7 @@ int lhb_paged_attention_q8_batched(lhb_ctx* ctx, const float* Q, const int8_t* K
     if (n_req < 0 || max_blocks <= 0 || n_req > 65535) return LHB_ERR_BAD_SHAPE;
     if (n_req == 0) return LHB_OK;
     cudaStream_t st = as_stream(stream);
-    if (decode_fast_ok(*cfg, *L) && aligned16(Q) && aligned16(Kp) && aligned16(Vp) &&
-        aligned16(Ks) && aligned16(Vs) && aligned16(O)) {
-        const int e = launch_decode_fast(ctx, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, n_req,
-                                         O, *cfg, *L, st);
-        if (e != LHB_ERR_SCRATCH) return e;
-    }
-    return launch_paged_attention_generic(ctx, true, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens,
-                                          0, n_req, O, *cfg, *L, st);
+    return dispatch_attn_q8(ctx, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, 0, n_req, O, *cfg, *L, st);
 }
 
 int lhb_paged_attention_q8(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp,
@@ -263,8 +269,8 @@ int lhb_paged_attention_q8(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const
     // the single-request form knows seq_len on the host; the table length it
     // implies is ceil(seq_len / block_size)
     const int max_blocks = std::max(1, ceil_div(seq_len, L->block_size));
-    return launch_paged_attention_generic(ctx, true, Q, Kp, Vp, Ks, Vs, table, max_blocks, nullptr,
-                                          seq_len, 1, O, *cfg, *L, as_stream(stream));
+    return dispatch_attn_q8(ctx, Q, Kp, Vp, Ks, Vs, table, max_blocks, nullptr, seq_len, 1, O, *cfg, *L,
+                            as_stream(stream));
 }
 
 int lhb_paged_attention_f32_batched(lhb_ctx* ctx, const float* Q, const float* Kp, const float* Vp,
@@ -275,6 +281,8 @@ int lhb_paged_attention_f32_batched(lhb_ctx* ctx, const float* Q, const float* K
     if (int e = check_attn(cfg, L)) return e;
     if (n_req < 0 || max_blocks <= 0 || n_req > 65535) return LHB_ERR_BAD_SHAPE;
     if (n_req == 0) return LHB_OK;
+    if (decode_f32_fast_ok(*cfg, *L) && aligned16(Q) && aligned16(Kp) && aligned16(Vp) && aligned16(O))
+        return launch_decode_f32_fast(ctx, Q, Kp, Vp, tables, max_blocks, seq_lens, n_req, O, *cfg, *L, as_stream(stream));
     return launch_paged_attention_generic(ctx, false, Q, Kp, Vp, nullptr, nullptr, tables, max_blocks,
                                           seq_lens, 0, n_req, O, *cfg, *L, as_stream(stream));
 }

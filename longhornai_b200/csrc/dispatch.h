@@ -41,10 +41,17 @@ int launch_w8a8_sharded(lhb_ctx* ctx, const int8_t* Aq, const int8_t* Bq, const 
 
 // split-KV decode attention (paged_attention_decode.cu)
 bool decode_fast_ok(const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L);
+// (seq_lens null: every request holds seq_len tokens)
 int launch_decode_fast(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp,
                        const float* Ks, const float* Vs, const int32_t* tables, int max_blocks,
-                       const int32_t* seq_lens, int n_req, float* O, const lhb_paged_attn_cfg& cfg,
+                       const int32_t* seq_lens, int seq_len, int n_req, float* O, const lhb_paged_attn_cfg& cfg,
                        const lhb_paged_layout& L, cudaStream_t st);
+
+// split-KV decode attention over fp32 pools (paged_attention_decode_f32.cu)
+bool decode_f32_fast_ok(const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L);
+int launch_decode_f32_fast(lhb_ctx* ctx, const float* Q, const float* Kp, const float* Vp, const int32_t* tables,
+                           int max_blocks, const int32_t* seq_lens, int n_req, float* O,
+                           const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L, cudaStream_t st);
 
 // W4A16 with a prologue on the activations (1 = RMSNorm with gamma/eps, 2 = SwiGLU of [gate || value] rows)
 // tensor-core W4A16 for a few rows up to a few hundred (gemm_w4a16_tc.cu); prologue 0 = none,

@@ -7,18 +7,20 @@
 // scale row.  The path is HBM-bound: every page is read once for the whole GQA
 // group (up to 4 query heads share a KV head).
 //
-// Work split: grid = (splits, kv heads, requests).  A CTA owns a contiguous
+// Work split: grid = (splits, kv heads x groups of four query heads, requests).  With more
+// than four query heads per KV head the neighbouring CTAs of a KV head read the same pages at
+// about the same time, so all but the first find them in L2.  A CTA owns a contiguous
 // range of the request's visible pages; its 4 warps take pages round-robin and
 // run independent cp.async rings (3 stages x 4.1 KiB per warp, 128-bit copies,
 // XOR-swizzled 16-byte chunks) -- no block-level barrier inside the main loop.
 // Per page a warp does, entirely on the int8 tensor-core path (mma.sync s8):
 //   S = K Q^T  : m16n8k32, tokens as the 16 rows, head_dim as k; the int8 rows of
 //                K are operand registers as they lie in shared memory (no
-//                conversion at all); Q is three signed 7-bit digits per element
+//                conversion at all); Q is three signed 7- or 8-bit digits per element
 //                (exact power-of-two scaling per head), one MMA column per digit;
 //   softmax in base 2 with the V row scale folded into the exponent:
 //                P = 2^(s*c + log2(vs) - m_ref) <= 1 whatever the magnitude of the
-//                scales, written as three 7-bit digits of round(2^20 P); the
+//                scales, written as three such digits of round(2^20 P) or round(2^22 P); the
 //                denominator is tracked in fp32 in the same frame;
 //   O += V^T P : m16n8k16 with head_dim as the 16 rows and the page's 16 tokens as
 //                k; 4x4 byte transposes (byte-permute) turn V rows into operand
@@ -34,7 +36,9 @@
 //
 // Results differ from the reference's three-pass softmax
 // (src/kernels/kvcache_quant.cpp:82-161) only by fp32 summation order and the
-// 2^-21 rounding of Q and P to 20-bit integers.
+// rounding of Q and P to integers: 2^-21 with 7-bit digits (the batched calls: 8e-6 of the
+// result's norm against fp64 for normal data), 2^-23 with 8-bit ones (the single-request call
+// and groups of more than four query heads, whose callers had fp32 sums before they ran here: 2e-6).  The time is the same.
 
 #include <cstdlib>
 #include <mutex>
@@ -62,7 +66,7 @@ constexpr int PD_WARP_BYTES = PD_STAGES * PD_STAGE_BYTES + 256;  // + P digit ex
 constexpr int PD_SMEM_BYTES = PD_WARPS * PD_WARP_BYTES + 2048;  // + the CTA's Q digit fragments
 constexpr int PD_MAX_GROUP = 4;
 constexpr int PD_PART = PD_D + 2;                               // floats per (split, head): m, l, O[128]
-constexpr float PD_WSHIFT = 20.0f;                              // P weights are integers in [0, 2^20]
+__host__ __device__ constexpr float pd_wshift(int bits) { return 3.0f * bits - (bits == 7 ? 1.0f : 2.0f); }   // P weights are integers in [0, 2^20] or [0, 2^22]
 constexpr float PD_MIN_LOG2_VS = -100.0f;
 constexpr float PD_FRAME_MARGIN = 3.0f;                         // head room of the integer frame, in log2 units
 
@@ -149,29 +153,44 @@ struct DecodeParams {
     const float* Ks;
     const float* Vs;
     const int32_t* tables;   // [n_req, max_blocks]
-    const int32_t* seq_lens; // [n_req]
+    const int32_t* seq_lens; // [n_req], or null: every request holds seq_len tokens
     float* O;
-    float* part;             // scratch: [n_req, n_kv, splits, group, PD_PART]
-    int* counters;           // [n_req * n_kv], zero between calls
+    float* part;             // scratch: [n_req, n_kv * subs, splits, min(group, 4), PD_PART]
+    int* counters;           // [n_req * n_kv * subs], zero between calls
     int* status;
+    int seq_len;
     int max_blocks, n_q_heads, n_kv_heads, group, num_blocks;
+    int subs;                // groups of up to four query heads per KV head
     int splits;              // grid.x: the most splits any request can use
     int pages_per_cta;       // a request is cut into ceil(pages / pages_per_cta) splits, at most `splits`
     int window, chunk;
     float scale_log2e;
 };
 
+// the lowest signed digit of BITS bits
+template <int BITS>
+__device__ __forceinline__ int pd_low_digit(int v) {
+    return BITS == 8 ? static_cast<int>(static_cast<int8_t>(v)) : ((v + 64) & 127) - 64;
+}
+
+template <int BITS>
 __global__ void __launch_bounds__(PD_THREADS, LHB_PD_MIN_CTAS)
 paged_decode_q8_kernel(const DecodeParams p) {
+    constexpr float R1 = static_cast<float>(1 << BITS), R2 = R1 * R1;       // weights of the digits
+    constexpr float WSHIFT = pd_wshift(BITS);
+    constexpr float QLIM = BITS == 8 ? 4194304.0f : 1048576.0f;
     extern __shared__ __align__(128) uint8_t pd_smem[];
     __shared__ int s_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int split = blockIdx.x, kvh = blockIdx.y, req = blockIdx.z;
-    const int G = p.group;
+    const int split = blockIdx.x, req = blockIdx.z;
+    const int kvh = blockIdx.y / p.subs, sub = blockIdx.y - kvh * p.subs;
+    const int G = min(PD_MAX_GROUP, p.group - sub * PD_MAX_GROUP);      // query heads of this CTA, from head0 on
+    const int GP = min(PD_MAX_GROUP, p.group);                          // heads per slot of the partials
+    const int head0 = kvh * p.group + sub * PD_MAX_GROUP;
 
     // ---- visible key range of the single query row (seq_q == 1) -------------
-    int len = p.seq_lens[req];
+    int len = p.seq_lens ? p.seq_lens[req] : p.seq_len;
     len = max(0, min(len, p.max_blocks * PD_BS));
     const int last = len - 1;
     int first = 0;
@@ -188,8 +207,8 @@ paged_decode_q8_kernel(const DecodeParams p) {
     const int pg_hi = min(page_f + n_pages, pg_lo + per_split);   // exclusive
     const int32_t* table = p.tables + static_cast<int64_t>(req) * p.max_blocks;
 
-    // ---- Q as three signed 7-bit digits per element (q*s = d1*2^14 + d2*2^7 + d3, s a
-    // power of two per head putting max|q| in [2^19, 2^20)), one int8 MMA column per
+    // ---- Q as three signed digits per element (q*s = d1*2^2b + d2*2^b + d3, b = BITS, s a
+    // power of two per head putting max|q| in [2^21, 2^22), or [2^19, 2^20) for b = 7), one int8 MMA column per
     // digit.  Column layout of the two 8-column operand blocks: block 0 column 2h = d1,
     // 2h+1 = d2 of head h; block 1 column 2h = d3 (odd columns zero), so thread (g, t)
     // of the result fragment owns every digit of head t.  Thread (g, t) of the operand
@@ -198,7 +217,7 @@ paged_decode_q8_kernel(const DecodeParams p) {
     uint32_t qf[4][2][2];            // [k-step][block][register]
     float qinv[PD_MAX_GROUP];
     {
-        const float* qbase = p.Q + (static_cast<int64_t>(req) * p.n_q_heads + kvh * G) * PD_D;
+        const float* qbase = p.Q + (static_cast<int64_t>(req) * p.n_q_heads + head0) * PD_D;
 #pragma unroll
         for (int h = 0; h < PD_MAX_GROUP; ++h) {
             float mx = 0.0f;
@@ -208,7 +227,7 @@ paged_decode_q8_kernel(const DecodeParams p) {
             }
             mx = warp_max(mx);
             const int e = static_cast<int>((__float_as_uint(mx) >> 23) & 0xff);
-            int se = (mx > 0.0f) ? 273 - e : 127;          // 127 + 19 - (e - 127)
+            int se = (mx > 0.0f) ? (BITS == 8 ? 275 : 273) - e : 127;          // 127 + 21 (19) - (e - 127)
             se = max(1, min(253, se));
             qinv[h] = __uint_as_float(static_cast<uint32_t>(254 - se) << 23);
         }
@@ -229,11 +248,11 @@ paged_decode_q8_kernel(const DecodeParams p) {
                 uint32_t b0 = 0, b1 = 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    int iv = __float2int_rn(fminf(fmaxf(x[j], -1048576.0f), 1048576.0f));
-                    const int lo = ((iv + 64) & 127) - 64;
-                    iv = (iv - lo) >> 7;
-                    const int mid = ((iv + 64) & 127) - 64;
-                    const int hi = (iv - mid) >> 7;
+                    int iv = __float2int_rn(fminf(fmaxf(x[j], -QLIM), QLIM));
+                    const int lo = pd_low_digit<BITS>(iv);
+                    iv = (iv - lo) >> BITS;
+                    const int mid = pd_low_digit<BITS>(iv);
+                    const int hi = (iv - mid) >> BITS;
                     b0 |= static_cast<uint32_t>((odd ? mid : hi) & 0xff) << (8 * j);
                     b1 |= static_cast<uint32_t>((odd ? 0 : lo) & 0xff) << (8 * j);
                 }
@@ -274,10 +293,10 @@ paged_decode_q8_kernel(const DecodeParams p) {
     auto fold = [&](float alpha) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const float a = fmaf(16384.0f, __int2float_rn(oi0[i][0]),
-                                 fmaf(128.0f, __int2float_rn(oi0[i][1]), __int2float_rn(oi1[i][0])));
-            const float b = fmaf(16384.0f, __int2float_rn(oi0[i][2]),
-                                 fmaf(128.0f, __int2float_rn(oi0[i][3]), __int2float_rn(oi1[i][2])));
+            const float a = fmaf(R2, __int2float_rn(oi0[i][0]),
+                                 fmaf(R1, __int2float_rn(oi0[i][1]), __int2float_rn(oi1[i][0])));
+            const float b = fmaf(R2, __int2float_rn(oi0[i][2]),
+                                 fmaf(R1, __int2float_rn(oi0[i][3]), __int2float_rn(oi1[i][2])));
             of[i][0] = (of[i][0] + a) * alpha;
             of[i][1] = (of[i][1] + b) * alpha;
             oi0[i][0] = oi0[i][1] = oi0[i][2] = oi0[i][3] = 0;
@@ -363,8 +382,8 @@ paged_decode_q8_kernel(const DecodeParams p) {
         }
         // ---- scores in base 2, V row scale folded into the exponent ------------------------
         const uint32_t sca = st + 4096 + 4 * g;               // ks[g], +32: ks[g+8], +64: vs[g], +96: vs[g+8]
-        float x0 = fmaf(16384.0f, pd_i2f(s0[0]), fmaf(128.0f, pd_i2f(s0[1]), pd_i2f(s1[0]))) * ldsf(sca) * sc;
-        float x1 = fmaf(16384.0f, pd_i2f(s0[2]), fmaf(128.0f, pd_i2f(s0[3]), pd_i2f(s1[2]))) * ldsf(sca + 32) * sc;
+        float x0 = fmaf(R2, pd_i2f(s0[0]), fmaf(R1, pd_i2f(s0[1]), pd_i2f(s1[0]))) * ldsf(sca) * sc;
+        float x1 = fmaf(R2, pd_i2f(s0[2]), fmaf(R1, pd_i2f(s0[3]), pd_i2f(s1[2]))) * ldsf(sca + 32) * sc;
         const int p0 = tok0 + g, p1 = tok0 + g + 8;
         const bool ok0 = page_ok && p0 >= first && p0 <= last;
         const bool ok1 = page_ok && p1 >= first && p1 <= last;
@@ -380,7 +399,7 @@ paged_decode_q8_kernel(const DecodeParams p) {
         // The int32 sums are kept in the frame of m_ref.  When a head's maximum rises
         // above it, the sums are folded into fp32 and the frame moves to the new
         // maximum plus a margin of 3 (weights then start at <= 2^-3 of full scale,
-        // still 17 bits), so that later, smaller rises need no fold; a sequence
+        // still 17 or 19 bits), so that later, smaller rises need no fold; a sequence
         // usually folds once.  Every 4096 pages a fold keeps the int32 sums in range.
         const bool rise = mp > m_ref;
         if (__any_sync(0xffffffffu, rise) || pages_since_fold == 4096) {
@@ -394,15 +413,15 @@ paged_decode_q8_kernel(const DecodeParams p) {
         ++pages_since_fold;
         const float mb = (m_ref == -INFINITY) ? 0.0f : m_ref;
         l_run += fast_exp2(x0 - mb) + fast_exp2(x1 - mb);
-        // ---- P = 2^20 * 2^(y - m_ref) <= 2^20 as three 7-bit digits, through shared memory
+        // ---- P = 2^WSHIFT * 2^(y - m_ref) as three digits, through shared memory
         // into operand order: column c of a block, tokens 4t .. 4t+3 in one register
         {
-            int w0 = __float2int_rn(fast_exp2(y0 - mb + PD_WSHIFT));
-            int w1 = __float2int_rn(fast_exp2(y1 - mb + PD_WSHIFT));
-            const int l0 = ((w0 + 64) & 127) - 64; w0 = (w0 - l0) >> 7;
-            const int l1 = ((w1 + 64) & 127) - 64; w1 = (w1 - l1) >> 7;
-            const int m0 = ((w0 + 64) & 127) - 64; const int h0 = (w0 - m0) >> 7;
-            const int m1 = ((w1 + 64) & 127) - 64; const int h1 = (w1 - m1) >> 7;
+            int w0 = __float2int_rn(fast_exp2(y0 - mb + WSHIFT));
+            int w1 = __float2int_rn(fast_exp2(y1 - mb + WSHIFT));
+            const int l0 = pd_low_digit<BITS>(w0); w0 = (w0 - l0) >> BITS;
+            const int l1 = pd_low_digit<BITS>(w1); w1 = (w1 - l1) >> BITS;
+            const int m0 = pd_low_digit<BITS>(w0); const int h0 = (w0 - m0) >> BITS;
+            const int m1 = pd_low_digit<BITS>(w1); const int h1 = (w1 - m1) >> BITS;
             // block 0 column 2t (d1) at +0, column 2t+1 (d2) at +16, block 1 column 2t (d3) at +128
             sts8(pst, h0); sts8(pst + 8, h1);
             sts8(pst + 16, m0); sts8(pst + 24, m1);
@@ -456,7 +475,8 @@ paged_decode_q8_kernel(const DecodeParams p) {
     }
     __syncthreads();
     const int d = threadIdx.x;                          // 128 threads <-> 128 head_dim elements
-    const int64_t pbase = ((static_cast<int64_t>(req) * p.n_kv_heads + kvh) * p.splits + split) * G;
+    const int cidx = req * static_cast<int>(gridDim.y) + static_cast<int>(blockIdx.y);
+    const int64_t pbase = (static_cast<int64_t>(cidx) * p.splits + split) * GP;
     for (int h = 0; h < G; ++h) {
         float M = -INFINITY;
 #pragma unroll
@@ -470,8 +490,8 @@ paged_decode_q8_kernel(const DecodeParams p) {
             o += f * sm_o[(w * PD_MAX_GROUP + h) * PD_D + d];
         }
         if (nsplit == 1) {
-            float* out = p.O + (static_cast<int64_t>(req) * p.n_q_heads + kvh * G + h) * PD_D;
-            out[d] = (L > 0.0f) ? o * (1.0f / L) * exp2f(-PD_WSHIFT) : 0.0f;
+            float* out = p.O + (static_cast<int64_t>(req) * p.n_q_heads + head0 + h) * PD_D;
+            out[d] = (L > 0.0f) ? o * (1.0f / L) * exp2f(-WSHIFT) : 0.0f;
         } else {
             float* pp = p.part + (pbase + h) * PD_PART;
             if (d == 0) { pp[0] = M; pp[1] = L; }
@@ -485,7 +505,6 @@ paged_decode_q8_kernel(const DecodeParams p) {
     // orders every thread's partial stores ahead of the fence, the barrier after it orders
     // the other splits' stores ahead of every thread's loads.
     __syncthreads();
-    const int cidx = req * p.n_kv_heads + kvh;
     if (threadIdx.x == 0) {
         __threadfence();
         const int old = atomicAdd(p.counters + cidx, 1);
@@ -501,7 +520,7 @@ paged_decode_q8_kernel(const DecodeParams p) {
     // eight splits are in flight together, so the merge costs one memory round trip per
     // eight splits instead of one per partial.  Splits are folded in split order with a
     // running maximum (deterministic).
-    const int64_t b0 = (static_cast<int64_t>(req) * p.n_kv_heads + kvh) * p.splits * G;
+    const int64_t b0 = static_cast<int64_t>(cidx) * p.splits * GP;
     const int mw = threadIdx.x >> 5, ml = threadIdx.x & 31;
     for (int h = mw; h < G; h += PD_WARPS) {
         float M = -INFINITY, L = 0.0f;
@@ -514,7 +533,7 @@ paged_decode_q8_kernel(const DecodeParams p) {
                 ms[j] = -INFINITY; ls[j] = 0.0f;
                 va[j] = make_float2(0.f, 0.f); vb[j] = make_float2(0.f, 0.f);
                 if (s0 + j < nsplit) {
-                    const float* pp = p.part + (b0 + (s0 + j) * G + h) * PD_PART;
+                    const float* pp = p.part + (b0 + (s0 + j) * GP + h) * PD_PART;
                     ms[j] = __ldcg(pp);
                     ls[j] = __ldcg(pp + 1);
                     va[j] = __ldcg(reinterpret_cast<const float2*>(pp + 2 + 2 * ml));
@@ -535,8 +554,8 @@ paged_decode_q8_kernel(const DecodeParams p) {
             }
             M = Mb;
         }
-        float* out = p.O + (static_cast<int64_t>(req) * p.n_q_heads + kvh * G + h) * PD_D;
-        const float r = (L > 0.0f) ? (1.0f / L) * exp2f(-PD_WSHIFT) : 0.0f;
+        float* out = p.O + (static_cast<int64_t>(req) * p.n_q_heads + head0 + h) * PD_D;
+        const float r = (L > 0.0f) ? (1.0f / L) * exp2f(-WSHIFT) : 0.0f;
         *reinterpret_cast<float2*>(out + 2 * ml) = make_float2(oa.x * r, oa.y * r);
         *reinterpret_cast<float2*>(out + 64 + 2 * ml) = make_float2(ob.x * r, ob.y * r);
     }
@@ -573,37 +592,42 @@ bool decode_fast_ok(const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L) {
     if (cfg.seq_q != 1 || cfg.head_dim != PD_D || L.head_dim != PD_D || L.block_size != PD_BS) return false;
     if (cfg.n_kv_heads <= 0 || cfg.n_q_heads % cfg.n_kv_heads) return false;
     const int group = cfg.n_q_heads / cfg.n_kv_heads;
-    return group >= 1 && group <= PD_MAX_GROUP && cfg.n_kv_heads <= 65535;
+    return group >= 1 && static_cast<int64_t>(cfg.n_kv_heads) * ceil_div(group, PD_MAX_GROUP) <= 65535;
 }
 
 int launch_decode_fast(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp,
                        const float* Ks, const float* Vs, const int32_t* tables, int max_blocks,
-                       const int32_t* seq_lens, int n_req, float* O, const lhb_paged_attn_cfg& cfg,
+                       const int32_t* seq_lens, int seq_len, int n_req, float* O, const lhb_paged_attn_cfg& cfg,
                        const lhb_paged_layout& L, cudaStream_t st) {
-    const int group = cfg.n_q_heads / cfg.n_kv_heads;
-    const int64_t items = static_cast<int64_t>(n_req) * cfg.n_kv_heads;
+    const int group = cfg.n_q_heads / cfg.n_kv_heads, subs = ceil_div(group, PD_MAX_GROUP);
+    const int64_t items = static_cast<int64_t>(n_req) * cfg.n_kv_heads * subs;
     int splits = 1, pages = max_blocks;
     decode_split_plan(ctx->sm_count, items, max_blocks,
-                      items > static_cast<int64_t>(ctx->counters_len) ? 0 : ctx->scratch_bytes / sizeof(float), group,
-                      &splits, &pages);
+                      items > static_cast<int64_t>(ctx->counters_len) ? 0 : ctx->scratch_bytes / sizeof(float),
+                      std::min(group, PD_MAX_GROUP), &splits, &pages);
     DecodeParams p{};
     p.Q = Q; p.Kp = Kp; p.Vp = Vp; p.Ks = Ks; p.Vs = Vs; p.tables = tables; p.seq_lens = seq_lens;
     p.O = O; p.part = reinterpret_cast<float*>(ctx->scratch); p.counters = ctx->counters;
     p.status = ctx->status_word;
     p.max_blocks = max_blocks; p.n_q_heads = cfg.n_q_heads; p.n_kv_heads = cfg.n_kv_heads;
-    p.group = group; p.num_blocks = L.num_blocks; p.splits = splits; p.pages_per_cta = pages;
+    p.group = group; p.subs = subs; p.seq_len = seq_len;
+    p.num_blocks = L.num_blocks; p.splits = splits; p.pages_per_cta = pages;
     p.window = cfg.window; p.chunk = cfg.chunk;
     const float scale = cfg.scale > 0.0f ? cfg.scale : 1.0f / sqrtf(static_cast<float>(cfg.head_dim));
     p.scale_log2e = scale * 1.4426950408889634f;
     const size_t smem = PD_SMEM_BYTES;
+    // a request on its own, or more than four query heads per KV head: 8-bit digits (see the top of the file)
+    auto kern = seq_lens && group <= PD_MAX_GROUP ? paged_decode_q8_kernel<7> : paged_decode_q8_kernel<8>;
     static bool attr_set[64] = {};
     if (!attr_set[ctx->device & 63]) {
-        LHB_CUDA(cudaFuncSetAttribute(paged_decode_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        LHB_CUDA(cudaFuncSetAttribute(paged_decode_q8_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(smem)));
+        LHB_CUDA(cudaFuncSetAttribute(paged_decode_q8_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(smem)));
         attr_set[ctx->device & 63] = true;
     }
-    dim3 grid(splits, cfg.n_kv_heads, n_req);
-    paged_decode_q8_kernel<<<grid, PD_THREADS, smem, st>>>(p);
+    dim3 grid(splits, cfg.n_kv_heads * subs, n_req);
+    kern<<<grid, PD_THREADS, smem, st>>>(p);
     LHB_LAUNCH_CHECK();
     return LHB_OK;
 }
@@ -659,7 +683,7 @@ int na_setup(int dev, NoAllocDevice** out) {
         LHB_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&d.counters), g_na_counters));
         LHB_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&d.status), g_na_status));
         LHB_CUDA(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
-        LHB_CUDA(cudaFuncSetAttribute(paged_decode_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        LHB_CUDA(cudaFuncSetAttribute(paged_decode_q8_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       PD_SMEM_BYTES));
         d.ready = true;
     }
@@ -683,7 +707,7 @@ extern "C" int lhb_paged_attention_q8_batched_noalloc(
     if (cfg->head_dim != layout->head_dim || cfg->n_kv_heads != layout->n_kv_heads || cfg->window < 0 ||
         cfg->chunk < 0 || cfg->n_q_heads <= 0)
         return LHB_ERR_BAD_SHAPE;
-    if (!decode_fast_ok(*cfg, *layout)) {
+    if (!decode_fast_ok(*cfg, *layout) || cfg->n_q_heads > PD_MAX_GROUP * cfg->n_kv_heads) {
         set_last_error_text("lhb_paged_attention_q8_batched_noalloc: only the decode shape is served "
                             "(seq_q 1, head_dim 128, block_size 16, at most 4 query heads per KV head)");
         return LHB_ERR_UNSUPPORTED;
@@ -721,12 +745,12 @@ extern "C" int lhb_paged_attention_q8_batched_noalloc(
     p.tables = block_tables; p.seq_lens = seq_lens; p.O = O;
     p.part = d->partials; p.counters = d->counters; p.status = d->status;
     p.max_blocks = max_blocks_per_req; p.n_q_heads = cfg->n_q_heads; p.n_kv_heads = cfg->n_kv_heads;
-    p.group = group; p.num_blocks = layout->num_blocks; p.splits = splits; p.pages_per_cta = pages;
+    p.group = group; p.subs = 1; p.num_blocks = layout->num_blocks; p.splits = splits; p.pages_per_cta = pages;
     p.window = cfg->window; p.chunk = cfg->chunk;
     const float scale = cfg->scale > 0.0f ? cfg->scale : 1.0f / sqrtf(static_cast<float>(cfg->head_dim));
     p.scale_log2e = scale * 1.4426950408889634f;
     dim3 grid(splits, cfg->n_kv_heads, n_requests);
-    paged_decode_q8_kernel<<<grid, PD_THREADS, PD_SMEM_BYTES, st>>>(p);
+    paged_decode_q8_kernel<7><<<grid, PD_THREADS, PD_SMEM_BYTES, st>>>(p);
     LHB_LAUNCH_CHECK();
     return LHB_OK;
 }

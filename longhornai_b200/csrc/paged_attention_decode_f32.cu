@@ -1,0 +1,314 @@
+// Split-KV paged decode attention over fp32 pages (seq_q == 1, head_dim 128, 16-token pages):
+// lh::paged_attention_batched (src/kernels/paged_attention.cpp:36-148) for the unquantised cache.
+//
+// HBM-bound: a page of one head is 8 KiB of K and 8 KiB of V, contiguous, read once for up to four query
+// heads.  Grid = (pieces of the longest table row, kv heads x groups of four query heads, requests);
+// requests shorter than the table use fewer pieces.  Eight warps take half-pages (8 tokens, 8 KiB)
+// round-robin through rings of three cp.async stages of their own, so 128 KiB per SM are in flight and the
+// main loop has no block barrier.  Scores: eight lanes share a token (16 dims each), so that a
+// head's dot product costs three shuffles per four tokens; the weighted sum: a lane owns four dims of
+// every head and reads the weights back from shared memory as one float4 per token.  All
+// arithmetic is fp32; about 370 instructions per 8 KiB, a third of the issue slots at the HBM rate.
+// Warps merge through shared memory, pieces through scratch by the last CTA to arrive, in order.
+// 8 requests of 256..2048 tokens, 32/8 heads (76 MB): 18.7 us; one CTA per query head and row needed 1450 us.
+#include <algorithm>
+
+#include "common.cuh"
+#include "dispatch.h"
+
+namespace lhb {
+
+constexpr int DF_D = 128, DF_BS = 16, DF_GROUP = 4;
+constexpr int DF_WARPS = 8, DF_THREADS = DF_WARPS * 32;
+constexpr int DF_TOK = 8;                                     // tokens of a stage
+constexpr int DF_STAGES = 3;
+constexpr int DF_STAGE_FLOATS = 2 * DF_TOK * DF_D;            // K rows, then V rows
+constexpr int DF_WARP_FLOATS = DF_STAGES * DF_STAGE_FLOATS + DF_TOK * DF_GROUP;   // + weights [token][head]
+constexpr int DF_SMEM = DF_WARPS * DF_WARP_FLOATS * 4;
+constexpr int DF_PART = DF_D + 2;                             // floats per (piece, head): O[128], m, l
+
+struct DecodeF32Params {
+    const float* Q;
+    const float* Kp;
+    const float* Vp;
+    const int32_t* tables;
+    const int32_t* seq_lens;
+    float* O;
+    float* part;             // [n_req][y][pieces][min(group, 4)][DF_PART]
+    int* counters;           // [n_req][y], zero between calls
+    int max_blocks, num_blocks, n_q_heads, n_kv_heads, group, subs;
+    int pieces, pages_per_cta;
+    int window, chunk;
+    float scale_log2e;
+};
+
+__device__ __forceinline__ void df_copy16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ float df_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// weight of a partial with maximum m in the frame M (M >= m); a partial without keys has none
+__device__ __forceinline__ float df_weight(float m, float M) { return m == -INFINITY ? 0.0f : df_exp2(m - M); }
+
+__global__ void __launch_bounds__(DF_THREADS, 1) paged_decode_f32_kernel(const DecodeF32Params p) {
+    extern __shared__ __align__(128) float df_smem[];
+    __shared__ float sm_ml[DF_WARPS][DF_GROUP][2];
+    __shared__ int s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tq = lane >> 3, dl = lane & 7;                  // token of a group of four, sixteenth of its row
+    const int piece = blockIdx.x, req = blockIdx.z;
+    const int kvh = blockIdx.y / p.subs, sub = blockIdx.y - kvh * p.subs;
+    const int G = min(DF_GROUP, p.group - sub * DF_GROUP), GP = min(DF_GROUP, p.group);
+    const int head0 = kvh * p.group + sub * DF_GROUP;
+
+    const int len = max(0, min(p.seq_lens[req], p.max_blocks * DF_BS));
+    const int last = len - 1;
+    int first = 0;
+    if (p.window > 0) first = max(0, len - p.window);
+    if (p.chunk > 0 && len > 0) first = max(first, (last / p.chunk) * p.chunk);
+    const int page_f = first / DF_BS;
+    const int n_pages = len > 0 ? last / DF_BS - page_f + 1 : 0;
+    const int np = max(1, min(p.pieces, (n_pages + p.pages_per_cta - 1) / p.pages_per_cta));
+    if (piece >= np) return;
+    const int per = (n_pages + np - 1) / np;
+    const int pg_lo = page_f + piece * per, pg_hi = min(page_f + n_pages, pg_lo + per);
+    const int32_t* table = p.tables + static_cast<int64_t>(req) * p.max_blocks;
+
+    // Q of up to four heads: this lane's four float4s of each (4 dl + 32 i), scaled to base-2 scores
+    float4 q[DF_GROUP][4];
+#pragma unroll
+    for (int h = 0; h < DF_GROUP; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (h < G) v = *reinterpret_cast<const float4*>(p.Q + (static_cast<int64_t>(req) * p.n_q_heads + head0 + h) * DF_D + 4 * dl + 32 * i);
+            q[h][i] = make_float4(v.x * p.scale_log2e, v.y * p.scale_log2e, v.z * p.scale_log2e, v.w * p.scale_log2e);
+        }
+
+    float* ring = df_smem + warp * DF_WARP_FLOATS;
+    float* wts = ring + DF_STAGES * DF_STAGE_FLOATS;
+    const uint32_t ring_u = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
+    // this warp's half-pages: it = 2 * (page index of the warp) + half, pages pg_lo + warp, + 8, ...
+    const int my_pages = pg_hi > pg_lo + warp ? (pg_hi - pg_lo - warp + DF_WARPS - 1) / DF_WARPS : 0;
+    const int n_it = 2 * my_pages;
+    int32_t ids = 0;                                          // lane l: page id of the warp's page 32 * batch + l
+    int batch = -1;
+    auto page_id = [&](int it) {                              // calls come in order of `it`
+        const int pi = it >> 1;
+        if ((pi >> 5) != batch) {
+            batch = pi >> 5;
+            const int i = batch * 32 + lane;
+            ids = i < my_pages ? table[pg_lo + warp + i * DF_WARPS] : -1;
+        }
+        const int blk = __shfl_sync(0xffffffffu, ids, pi & 31);
+        return (blk >= 0 && blk < p.num_blocks) ? blk : -1;   // a bad id is never dereferenced; its keys are masked
+    };
+    uint32_t ok_bits = 0;                                     // bit it & 31: the page of iteration it is valid
+    auto issue = [&](int it) {
+        if (it < n_it) {
+            const int blk = page_id(it);
+            ok_bits = blk >= 0 ? (ok_bits | (1u << (it & 31))) : (ok_bits & ~(1u << (it & 31)));
+            const int64_t row = (static_cast<int64_t>(max(blk, 0)) * p.n_kv_heads + kvh) * DF_BS + (it & 1) * DF_TOK;
+            const float* k = p.Kp + row * DF_D + lane * 4;
+            const float* v = p.Vp + row * DF_D + lane * 4;
+            const uint32_t dst = ring_u + ((it % DF_STAGES) * DF_STAGE_FLOATS + lane * 4) * 4;
+#pragma unroll
+            for (int i = 0; i < DF_TOK; ++i) {
+                df_copy16(dst + i * DF_D * 4, k + i * DF_D);
+                df_copy16(dst + (DF_TOK + i) * DF_D * 4, v + i * DF_D);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int s = 0; s < DF_STAGES - 1; ++s) issue(s);
+
+    float m[DF_GROUP], l[DF_GROUP];                           // running maximum (same on all lanes), this lane's share of the sum
+    float4 o[DF_GROUP];
+#pragma unroll
+    for (int h = 0; h < DF_GROUP; ++h) { m[h] = -INFINITY; l[h] = 0.0f; o[h] = make_float4(0.f, 0.f, 0.f, 0.f); }
+
+    for (int it = 0; it < n_it; ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DF_STAGES - 2) : "memory");
+        __syncwarp();                                         // every lane's copies have landed; iteration it - 1 is done
+        const bool page_ok = (ok_bits >> (it & 31)) & 1u;
+        issue(it + DF_STAGES - 1);
+        const float* st = ring + (it % DF_STAGES) * DF_STAGE_FLOATS;
+        const int tok0 = (pg_lo + warp + (it >> 1) * DF_WARPS) * DF_BS + (it & 1) * DF_TOK;
+        float s[2][DF_GROUP];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {                         // tokens 4u + tq
+            const float* kr = st + (4 * u + tq) * DF_D + 4 * dl;
+            float4 k[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) k[i] = *reinterpret_cast<const float4*>(kr + 32 * i);
+            const int pos = tok0 + 4 * u + tq;
+            const bool ok = page_ok && pos >= first && pos <= last;
+#pragma unroll
+            for (int h = 0; h < DF_GROUP; ++h) {
+                float d0 = 0.0f, d1 = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    d0 = fmaf(q[h][i].x, k[i].x, d0); d0 = fmaf(q[h][i].y, k[i].y, d0);
+                    d0 = fmaf(q[h][i].z, k[i].z, d0); d0 = fmaf(q[h][i].w, k[i].w, d0);
+                    d1 = fmaf(q[h][i + 1].x, k[i + 1].x, d1); d1 = fmaf(q[h][i + 1].y, k[i + 1].y, d1);
+                    d1 = fmaf(q[h][i + 1].z, k[i + 1].z, d1); d1 = fmaf(q[h][i + 1].w, k[i + 1].w, d1);
+                }
+                float d = d0 + d1;
+                d += __shfl_xor_sync(0xffffffffu, d, 1);
+                d += __shfl_xor_sync(0xffffffffu, d, 2);
+                d += __shfl_xor_sync(0xffffffffu, d, 4);
+                s[u][h] = ok ? d : -INFINITY;
+            }
+        }
+        float w0 = 0.0f, w1 = 0.0f;                           // lanes dl < 4: the weights of head dl for this lane's tokens
+#pragma unroll
+        for (int h = 0; h < DF_GROUP; ++h) {
+            float mx = fmaxf(s[0][h], s[1][h]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            const float mn = fmaxf(m[h], mx);
+            const float a = m[h] == mn ? 1.0f : df_exp2(m[h] - mn);      // exp2(-inf) = 0
+            const float mb = mn == -INFINITY ? 0.0f : mn;
+            const float p0 = df_exp2(s[0][h] - mb), p1 = df_exp2(s[1][h] - mb);
+            m[h] = mn;
+            l[h] = fmaf(l[h], a, p0 + p1);
+            o[h].x *= a; o[h].y *= a; o[h].z *= a; o[h].w *= a;
+            if (dl == h) { w0 = p0; w1 = p1; }
+        }
+        if (dl < DF_GROUP) { wts[tq * DF_GROUP + dl] = w0; wts[(4 + tq) * DF_GROUP + dl] = w1; }
+        __syncwarp();
+        const float* vr = st + DF_TOK * DF_D + 4 * lane;
+#pragma unroll
+        for (int i = 0; i < DF_TOK; ++i) {
+            const float4 w = *reinterpret_cast<const float4*>(wts + i * DF_GROUP);
+            float4 v = *reinterpret_cast<const float4*>(vr + i * DF_D);
+            // a masked token's row may hold anything (an unwritten slot): 0 * it must not be NaN
+            const int pos = tok0 + i;
+            if (!(page_ok && pos >= first && pos <= last)) v = make_float4(0.f, 0.f, 0.f, 0.f);
+            o[0].x = fmaf(w.x, v.x, o[0].x); o[0].y = fmaf(w.x, v.y, o[0].y); o[0].z = fmaf(w.x, v.z, o[0].z); o[0].w = fmaf(w.x, v.w, o[0].w);
+            o[1].x = fmaf(w.y, v.x, o[1].x); o[1].y = fmaf(w.y, v.y, o[1].y); o[1].z = fmaf(w.y, v.z, o[1].z); o[1].w = fmaf(w.y, v.w, o[1].w);
+            o[2].x = fmaf(w.z, v.x, o[2].x); o[2].y = fmaf(w.z, v.y, o[2].y); o[2].z = fmaf(w.z, v.z, o[2].z); o[2].w = fmaf(w.z, v.w, o[2].w);
+            o[3].x = fmaf(w.w, v.x, o[3].x); o[3].y = fmaf(w.w, v.y, o[3].y); o[3].z = fmaf(w.w, v.z, o[3].z); o[3].w = fmaf(w.w, v.w, o[3].w);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                          // rings are dead from here on
+    float* sm_o = df_smem;                                    // [warp][head][128]
+#pragma unroll
+    for (int h = 0; h < DF_GROUP; ++h) {
+        float ls = l[h];                                      // the eight lanes of a token hold the same share
+        ls += __shfl_xor_sync(0xffffffffu, ls, 8);
+        ls += __shfl_xor_sync(0xffffffffu, ls, 16);
+        if (lane == 0) { sm_ml[warp][h][0] = m[h]; sm_ml[warp][h][1] = ls; }
+        *reinterpret_cast<float4*>(sm_o + (warp * DF_GROUP + h) * DF_D + 4 * lane) = o[h];
+    }
+    __syncthreads();
+    const int cidx = req * static_cast<int>(gridDim.y) + static_cast<int>(blockIdx.y);
+    float* part = p.part + static_cast<int64_t>(cidx) * p.pieces * GP * DF_PART;
+    for (int h = warp; h < G; h += DF_WARPS) {                // one warp per head, four dims per lane
+        float M = -INFINITY, L = 0.0f;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int w = 0; w < DF_WARPS; ++w) M = fmaxf(M, sm_ml[w][h][0]);
+        for (int w = 0; w < DF_WARPS; ++w) {
+            const float f = df_weight(sm_ml[w][h][0], M);
+            const float4 v = *reinterpret_cast<const float4*>(sm_o + (w * DF_GROUP + h) * DF_D + 4 * lane);
+            L = fmaf(f, sm_ml[w][h][1], L);
+            r.x = fmaf(f, v.x, r.x); r.y = fmaf(f, v.y, r.y); r.z = fmaf(f, v.z, r.z); r.w = fmaf(f, v.w, r.w);
+        }
+        if (np == 1) {
+            const float inv = L == 0.0f ? 0.0f : __fdiv_rn(1.0f, L);
+            *reinterpret_cast<float4*>(p.O + (static_cast<int64_t>(req) * p.n_q_heads + head0 + h) * DF_D + 4 * lane) =
+                make_float4(r.x * inv, r.y * inv, r.z * inv, r.w * inv);
+        } else {
+            float* d = part + (piece * GP + h) * DF_PART;
+            *reinterpret_cast<float2*>(d + 4 * lane) = make_float2(r.x, r.y);
+            *reinterpret_cast<float2*>(d + 4 * lane + 2) = make_float2(r.z, r.w);
+            if (lane == 0) *reinterpret_cast<float2*>(d + DF_D) = make_float2(M, L);
+        }
+    }
+    if (np == 1) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {                                   // one fence for the CTA on either side of the count
+        __threadfence();
+        s_last = atomicAdd(p.counters + cidx, 1) == np - 1;
+        if (s_last) {
+            p.counters[cidx] = 0;                             // ready for the next call
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (!s_last) return;
+    for (int h = warp; h < G; h += DF_WARPS) {
+        float M = -INFINITY, L = 0.0f;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < np; s0 += 8) {                  // eight partials in flight
+            float2 ml[8], a[8], b[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float* d = part + (min(s0 + j, np - 1) * GP + h) * DF_PART;
+                ml[j] = __ldcg(reinterpret_cast<const float2*>(d + DF_D));
+                a[j] = __ldcg(reinterpret_cast<const float2*>(d + 4 * lane));
+                b[j] = __ldcg(reinterpret_cast<const float2*>(d + 4 * lane + 2));
+                if (s0 + j >= np) ml[j] = make_float2(-INFINITY, 0.0f);
+            }
+            float Mn = M;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) Mn = fmaxf(Mn, ml[j].x);
+            const float keep = df_weight(M, Mn);
+            L *= keep; r.x *= keep; r.y *= keep; r.z *= keep; r.w *= keep;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float f = df_weight(ml[j].x, Mn);
+                L = fmaf(f, ml[j].y, L);
+                r.x = fmaf(f, a[j].x, r.x); r.y = fmaf(f, a[j].y, r.y); r.z = fmaf(f, b[j].x, r.z); r.w = fmaf(f, b[j].y, r.w);
+            }
+            M = Mn;
+        }
+        const float inv = L == 0.0f ? 0.0f : __fdiv_rn(1.0f, L);
+        *reinterpret_cast<float4*>(p.O + (static_cast<int64_t>(req) * p.n_q_heads + head0 + h) * DF_D + 4 * lane) =
+            make_float4(r.x * inv, r.y * inv, r.z * inv, r.w * inv);
+    }
+}
+
+bool decode_f32_fast_ok(const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L) {
+    if (cfg.seq_q != 1 || cfg.head_dim != DF_D || L.head_dim != DF_D || L.block_size != DF_BS) return false;
+    return cfg.n_kv_heads > 0 && cfg.n_q_heads % cfg.n_kv_heads == 0 &&
+           static_cast<int64_t>(cfg.n_kv_heads) * ceil_div(cfg.n_q_heads / cfg.n_kv_heads, DF_GROUP) <= 65535;
+}
+
+int launch_decode_f32_fast(lhb_ctx* ctx, const float* Q, const float* Kp, const float* Vp, const int32_t* tables,
+                           int max_blocks, const int32_t* seq_lens, int n_req, float* O,
+                           const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L, cudaStream_t st) {
+    DecodeF32Params p{};
+    p.Q = Q; p.Kp = Kp; p.Vp = Vp; p.tables = tables; p.seq_lens = seq_lens; p.O = O;
+    p.part = reinterpret_cast<float*>(ctx->scratch); p.counters = ctx->counters;
+    p.max_blocks = max_blocks; p.num_blocks = L.num_blocks;
+    p.n_q_heads = cfg.n_q_heads; p.n_kv_heads = cfg.n_kv_heads; p.group = cfg.n_q_heads / cfg.n_kv_heads;
+    p.subs = ceil_div(p.group, DF_GROUP);
+    p.window = cfg.window; p.chunk = cfg.chunk;
+    const float scale = cfg.scale > 0.0f ? cfg.scale : 1.0f / sqrtf(static_cast<float>(cfg.head_dim));
+    p.scale_log2e = scale * 1.4426950408889634f;
+    // Pieces: about three CTAs per SM if every request were as long as the table (an SM holds one, and the
+    // shorter requests' missing pieces even the waves out), of at least one page per warp.
+    const int64_t items = static_cast<int64_t>(n_req) * p.n_kv_heads * p.subs;
+    const int64_t ppc = std::max<int64_t>(DF_WARPS, (items * max_blocks + 3 * ctx->sm_count - 1) / (3 * ctx->sm_count));
+    int64_t pieces = std::min<int64_t>(64, (max_blocks + ppc - 1) / ppc);
+    const size_t per_piece = static_cast<size_t>(items) * std::min(p.group, DF_GROUP) * DF_PART * sizeof(float);
+    if (items > static_cast<int64_t>(ctx->counters_len)) pieces = 1;
+    else if (pieces * per_piece > ctx->scratch_bytes) pieces = std::max<int64_t>(1, ctx->scratch_bytes / per_piece);
+    p.pieces = static_cast<int>(pieces);
+    p.pages_per_cta = ceil_div(max_blocks, p.pieces);
+    static bool attr_set[64] = {};
+    if (!attr_set[ctx->device & 63]) {
+        LHB_CUDA(cudaFuncSetAttribute(paged_decode_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DF_SMEM));
+        attr_set[ctx->device & 63] = true;
+    }
+    paged_decode_f32_kernel<<<dim3(p.pieces, p.n_kv_heads * p.subs, n_req), DF_THREADS, DF_SMEM, st>>>(p);
+    LHB_LAUNCH_CHECK();
+    return LHB_OK;
+}
+
+}  // namespace lhb
