@@ -233,14 +233,16 @@ static int check_attn(const lhb_paged_attn_cfg* cfg, const lhb_paged_layout* L) 
     return LHB_OK;
 }
 
-// One query row per request: split-KV decode kernel.  Several rows, other head dims, page sizes or
-// unaligned pointers: the generic kernel.
+// One query row per request: split-KV decode kernel.  Several: tensor-core prefill kernel.  Other head
+// dims, page sizes or unaligned pointers: the generic kernel.
 static int dispatch_attn_q8(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp, const float* Ks,
                             const float* Vs, const int32_t* tables, int max_blocks, const int32_t* seq_lens, int seq_len,
                             int n_req, float* O, const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L, cudaStream_t st) {
     if (aligned16(Q) && aligned16(Kp) && aligned16(Vp) && aligned16(Ks) && aligned16(Vs) && aligned16(O)) {
         if (decode_fast_ok(cfg, L))
             return launch_decode_fast(ctx, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, seq_len, n_req, O, cfg, L, st);
+        if (prefill_fast_ok(cfg, L))
+            return launch_prefill_fast(ctx, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, seq_len, n_req, O, cfg, L, st);
     }
     return launch_paged_attention_generic(ctx, true, Q, Kp, Vp, Ks, Vs, tables, max_blocks, seq_lens, seq_len, n_req, O,
                                           cfg, L, st);

@@ -53,6 +53,13 @@ int launch_decode_f32_fast(lhb_ctx* ctx, const float* Q, const float* Kp, const 
                            int max_blocks, const int32_t* seq_lens, int n_req, float* O,
                            const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L, cudaStream_t st);
 
+// several query rows per request over int8 pools, tcgen05 (paged_attention_prefill.cu)
+bool prefill_fast_ok(const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L);
+int launch_prefill_fast(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp, const float* Ks,
+                        const float* Vs, const int32_t* tables, int max_blocks, const int32_t* seq_lens,
+                        int seq_len_scalar, int n_req, float* O, const lhb_paged_attn_cfg& cfg,
+                        const lhb_paged_layout& L, cudaStream_t st);
+
 // W4A16 with a prologue on the activations (1 = RMSNorm with gamma/eps, 2 = SwiGLU of [gate || value] rows)
 // tensor-core W4A16 for a few rows up to a few hundred (gemm_w4a16_tc.cu); prologue 0 = none,
 // 1 = RMSNorm (gamma, eps), 2 = SwiGLU of [gate || value] rows.  w4a16_tc_min_rows: the row count

@@ -1,0 +1,596 @@
+// Prefill attention over int8 pages on the 5th-generation tensor cores: several query rows per
+// request (a prompt, or a chunk of one behind cached tokens), head_dim 128, 16-token pages.
+//
+// Semantics are those of the generic kernel (src/kernels/kvcache_quant.cpp:82-161: causal, window
+// and chunk masks, per-row K and V scales, no visible key = zeros).  The reference multiplies fp32
+// by dequantised int8, and tensor cores have no fp32 operands; int8 is exact in fp16, so both
+// contractions run as two kind::f16 passes over the high and the low half of the fp32 operand:
+//   S = (Qh + Ql) K^T   Q scaled by one power of two per CTA, split 11 + 11 bits;
+//   O += (Ph + Pl) V    P = 2^(s - m) * vs, split the same way: V stays the exact integers, its row scale
+//                       rides in the weight; l sums 2^(s - m).
+// P lives in a frame 2^F (F follows the largest V scale met) that fits fp16.  The tensor cores add to an fp32
+// accumulator with truncation, half an ulp per step and always towards zero: a whole prompt accumulated in
+// TMEM was off by 8.5e-6 at 4000 keys.  So an accumulator holds one tile of 128 keys only (16 steps)
+// and the running O is kept in registers, where it is rescaled and added to with rounding.
+//
+// A CTA takes 128 rows of one KV head: row R is query R / g, head R % g of the g query heads that
+// share the KV head, so a KV tile is converted once for the whole group.  S / P (P overwrites S in place) and O
+// are double-buffered in the 512 TMEM columns, K and V in shared memory, and the roles run free of each other:
+//   warps 0-7    softmax: 16 rows x 128 keys a warp.  A thread holds 2 rows x 32 keys in the fragment layout, so
+//                that a key's two scales are read once for two rows by an 8-byte load with four addresses a warp (the
+//                row-per-thread layout reads them with broadcasts, one wavefront per key, scale and warp:
+//                shared memory then is the bound), and adds the previous tile's O to its registers;
+//   warps 8-11   int8 -> fp16: 128-bit loads of whole pages straight to registers, one operand ahead, an
+//                exclusive-or, a byte permute and a subtraction per two values, 128-byte-swizzled stores.  K and V
+//                lie in shared memory as [token][d] alike, K read K-major, V MN-major;
+//   warp 12      MMA issuer: PV(j), then QK(j + 2) into the S it has freed.
+// What bounds it: per 128 x 128 tile 2048 tensor cycles, about 2300 cycles of shared-memory traffic (operands
+// 1536, conversion 512, scales 256) and about 2500 issue cycles (softmax 1700, conversion 670).
+// Few rows leave SMs idle: the keys are then split over CTAs and merged by a second small launch.
+//
+// Every wait is bounded (ptx::mbar_wait): a timeout sets the context's status word, the roles fall
+// through to the common exit and TMEM is freed.
+#include <algorithm>
+
+#include "common.cuh"
+#include "dispatch.h"
+#include "ptx.cuh"
+
+namespace lhb {
+
+constexpr int PF_D = 128, PF_BS = 16;
+constexpr int PF_ROWS = 128;                       // rows of a CTA
+constexpr int PF_KEYS = 128;                       // keys of a tile, eight pages
+constexpr int PF_TILE_BYTES = 128 * PF_D * 2;      // one fp16 operand tile: two 64-wide halves of 16 KiB
+constexpr int PF_HALF_BYTES = PF_TILE_BYTES / 2;
+constexpr int PF_THREADS = 16 * 32;                // four warpgroups: two softmax, converters, MMA issuer (and three idle warps)
+// Registers a thread after the split; the sum is what the launch allocates (4 x 128)
+constexpr int PF_REG_SOFTMAX = 192, PF_REG_CONVERT = 88, PF_REG_ISSUE = 40;
+static_assert(2 * PF_REG_SOFTMAX + PF_REG_CONVERT + PF_REG_ISSUE <= 4 * 128, "register split exceeds the launch");
+constexpr int PF_PARAM_FLOATS = 2 * PF_KEYS + 8;   // per tile: ks (times the scale of S), vs, then per 32 keys: largest vs (bits), validity bits
+constexpr int PF_PARAM_RING = 4;                   // the converters may be three tiles ahead of the softmax
+constexpr size_t PF_SMEM = 1024 + 6 * size_t(PF_TILE_BYTES) + PF_PARAM_RING * PF_PARAM_FLOATS * 4 + 256 + PF_ROWS;
+constexpr int PF_PART = PF_D + 2;                  // floats per (split, row): O[128], frame, l
+constexpr int PF_HEAD = 13;                        // P < 2^(HEAD + 1) in fp16
+constexpr int PF_MIN_FRAME = -60;                  // V scales below 2^-60 share a frame: 2^-frame must stay far from overflow
+
+struct PrefillParams {
+    const float* Q;
+    const int8_t* Kp;
+    const int8_t* Vp;
+    const float* Ks;
+    const float* Vs;
+    const int32_t* tables;
+    const int32_t* seq_lens;     // null: seq_len_scalar
+    float* O;
+    float* part;                 // [split][(req, kv head, row)][PF_PART]
+    int* status;
+    int seq_len_scalar, max_blocks, num_blocks;
+    int n_q_heads, n_kv_heads, group, seq_q;
+    int causal, window, chunk;
+    int splits, row_tiles;
+    int64_t total_rows;          // n_req * n_kv_heads * seq_q * group
+    float scale_log2e;
+};
+
+// D = f32 (bits 4-5 = 1), A = B = fp16 (0), B MN-major at bit 16, N >> 3 at bit 17, M >> 4 at bit 24
+constexpr uint32_t pf_idesc(bool b_mn) {
+    return (1u << 4) | (b_mn ? (1u << 16) : 0u) | (static_cast<uint32_t>(128 >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
+}
+
+__device__ __forceinline__ float pf_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// two fp32 -> packed fp16, `lo` in the low half
+__device__ __forceinline__ uint32_t pf_pack(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// four int8 -> two packed fp16 pairs: a byte b ^ 0x80 under the exponent byte 0x64 is 1024 + 128 + b
+__device__ __forceinline__ void pf_cvt4(uint32_t w, uint32_t& a, uint32_t& b) {
+    const uint32_t u = w ^ 0x80808080u;
+    a = __byte_perm(u, 0x64646464u, 0x4140);
+    b = __byte_perm(u, 0x64646464u, 0x4342);
+    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(a) : "r"(0x64806480u));
+    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(b) : "r"(0x64806480u));
+}
+// the part of |x| that fits fp16's 11 bits, by truncation; the rest is exact in fp32
+__device__ __forceinline__ float pf_high(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
+
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 pf_mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 pf_add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 pf_fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+    return d;
+}
+template <int N> __device__ __forceinline__ void pf_more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void pf_fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// keys [lo, hi] that the query at position `pos` sees (empty when lo > hi); lo and hi do not fall as pos rises
+__device__ __forceinline__ void pf_visible(const PrefillParams& p, int pos, int len, int& lo, int& hi) {
+    lo = 0;
+    hi = len - 1;
+    if (p.causal) hi = min(hi, pos);
+    if (p.window > 0) lo = max(lo, pos - p.window + 1);
+    if (p.chunk > 0) {
+        const int c = pos / p.chunk;               // truncated, as the reference's comparison of quotients
+        lo = max(lo, c * p.chunk);
+        hi = min(hi, c < 0 ? -1 : c * p.chunk + p.chunk - 1);
+    }
+}
+
+__global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const PrefillParams p) {
+    extern __shared__ uint8_t pf_smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pf_smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* q_sm = smem;                                        // high, low operand tile
+    uint8_t* k_sm = smem + 2 * PF_TILE_BYTES;                    // two tiles
+    uint8_t* v_sm = smem + 4 * PF_TILE_BYTES;                    // two tiles
+    float* par = reinterpret_cast<float*>(smem + 6 * PF_TILE_BYTES);                // [PF_PARAM_RING][PF_PARAM_FLOATS]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(par + PF_PARAM_RING * PF_PARAM_FLOATS);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    unsigned* q_max = tmem_slot + 2;                             // largest |q| of the CTA, bits
+    uint8_t* row_bad = reinterpret_cast<uint8_t*>(bars + 32);    // [PF_ROWS] rows with a NaN or an infinity
+    // barriers of buffer b = tile & 1: tile j waits for or completes phase j >> 1
+    const uint32_t bar0 = ptx::smem_u32(bars);
+    auto k_full = [&](int b) { return bar0 + 8 * b; };
+    auto k_empty = [&](int b) { return bar0 + 16 + 8 * b; };
+    auto v_full = [&](int b) { return bar0 + 32 + 8 * b; };
+    auto v_empty = [&](int b) { return bar0 + 48 + 8 * b; };
+    auto s_full = [&](int b) { return bar0 + 64 + 8 * b; };      // S is in TMEM
+    auto p_full = [&](int b) { return bar0 + 80 + 8 * b; };      // P is in TMEM
+    auto o_full = [&](int b) { return bar0 + 96 + 8 * b; };      // PV of the tile is in TMEM
+    auto o_free = [&](int b) { return bar0 + 112 + 8 * b; };     // and has been added to the registers
+    auto par_full = [&](int i) { return bar0 + 128 + 8 * i; };   // slot i = tile & 3: the scales of the tile, phase tile >> 2
+
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
+    const int g = p.group, kvh = blockIdx.y, req = blockIdx.z;
+    // later queries see more keys: longest rows first
+    const int rt = p.row_tiles - 1 - static_cast<int>(blockIdx.x) / p.splits, split = blockIdx.x % p.splits;
+    const int rows_all = p.seq_q * g;
+    const int r0 = rt * PF_ROWS, rows = min(PF_ROWS, rows_all - r0);
+    int len = p.seq_lens ? p.seq_lens[req] : p.seq_len_scalar;
+    len = max(0, min(len, p.max_blocks * PF_BS));
+    const int shift = len - p.seq_q;
+    const int32_t* table = p.tables + static_cast<int64_t>(req) * p.max_blocks;
+
+    int key_lo, key_hi, dummy;
+    pf_visible(p, shift + r0 / g, len, key_lo, dummy);
+    pf_visible(p, shift + (r0 + rows - 1) / g, len, dummy, key_hi);
+    const int page0 = key_lo / PF_BS;
+    const int tiles_all = key_hi >= key_lo ? (key_hi / PF_BS - page0 + 8) / 8 : 0;
+    const int j_lo = static_cast<int>(static_cast<int64_t>(tiles_all) * split / p.splits);
+    const int j_hi = static_cast<int>(static_cast<int64_t>(tiles_all) * (split + 1) / p.splits);
+    const int n_tiles = j_hi - j_lo;
+    const int page_base = page0 + j_lo * 8;                      // first page of this CTA's first tile
+
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; ++b) {
+            ptx::mbar_init(k_full(b), 128); ptx::mbar_init(k_empty(b), 1);
+            ptx::mbar_init(v_full(b), 128); ptx::mbar_init(v_empty(b), 1);
+            ptx::mbar_init(s_full(b), 1); ptx::mbar_init(p_full(b), 256);
+            ptx::mbar_init(o_full(b), 1); ptx::mbar_init(o_free(b), 256);
+        }
+        for (int i = 0; i < PF_PARAM_RING; ++i) ptx::mbar_init(par_full(i), 128);
+        *abort_flag = 0;
+        *q_max = 0;
+        ptx::fence_mbar_init();
+    }
+    if (warp == 12) {
+        ptx::tmem_alloc(ptx::smem_u32(tmem_slot), 512);
+        ptx::tmem_relinquish();
+    }
+    __syncthreads();
+    // ---- Q, one warp per 16 rows: the largest magnitude, then scale, split and store as two swizzled operand tiles ----
+    auto q_row = [&](int r) {
+        if (r >= rows) return make_float4(0.f, 0.f, 0.f, 0.f);
+        const int R = r0 + r, q = R / g, h = R - q * g;
+        return *reinterpret_cast<const float4*>(
+            p.Q + ((static_cast<int64_t>(req) * p.n_q_heads + kvh * g + h) * p.seq_q + q) * PF_D + lane * 4);
+    };
+    if (warp < 8) {
+        unsigned most = 0;
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+            const unsigned mb = __reduce_max_sync(0xffffffffu, abs_bits_max4(q_row(warp * 16 + i)));
+            if (lane == 0) row_bad[warp * 16 + i] = mb >= 0x7f800000u;
+            if (mb < 0x7f800000u) most = max(most, mb);
+        }
+        if (lane == 0) atomicMax(q_max, most);
+    }
+    __syncthreads();
+    // one power of two takes the CTA's largest |q| into [2^14, 2^15): a row 2^18 smaller still keeps 22 bits of its own maximum
+    int q_exp = *q_max ? 268 - static_cast<int>((*q_max >> 23) & 0xff) : 127;
+    q_exp = max(1, min(253, q_exp));
+    if (warp < 8) {
+        const float scl = __uint_as_float(static_cast<uint32_t>(q_exp) << 23);
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+            const int r = warp * 16 + i;
+            float4 v = q_row(r);
+            if (row_bad[r]) v = make_float4(0.f, 0.f, 0.f, 0.f);                  // the row's output becomes NaN at the end
+            v.x *= scl; v.y *= scl; v.z *= scl; v.w *= scl;
+            const float hx = pf_high(v.x), hy = pf_high(v.y), hz = pf_high(v.z), hw = pf_high(v.w);
+            // elements 4 * lane .. +3: half lane / 16, 16-byte chunk (lane % 16) / 2, 8 bytes into it
+            const int off = (lane >> 4) * PF_HALF_BYTES + r * 128 + (((((lane & 15) >> 1) ^ (r & 7))) << 4) + (lane & 1) * 8;
+            *reinterpret_cast<uint2*>(q_sm + off) = make_uint2(pf_pack(hx, hy), pf_pack(hz, hw));
+            *reinterpret_cast<uint2*>(q_sm + PF_TILE_BYTES + off) =
+                make_uint2(pf_pack(v.x - hx, v.y - hy), pf_pack(v.z - hz, v.w - hw));
+        }
+        ptx::fence_proxy_async_smem();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_slot;                            // columns: S / P buffers at 0 and 128, O buffers at 256 and 384
+
+    if (warp < 8) {
+        pf_more_registers<PF_REG_SOFTMAX>();
+        // ---- softmax: rows ra and ra + 8, columns 8 i + 2 (lane % 4) and + 1 ----
+        const int row16 = 32 * (warp & 3) + 16 * (warp >> 2);    // first of the warp's rows = TMEM lanes
+        const int ra = row16 + (lane >> 2), rb = ra + 8, col = 2 * (lane & 3);
+        const uint32_t base = tmem + (static_cast<uint32_t>(row16) << 16);
+        int lo_a = 0, hi_a = -1, lo_b = 0, hi_b = -1;
+        if (ra < rows) pf_visible(p, shift + (r0 + ra) / g, len, lo_a, hi_a);
+        if (rb < rows) pf_visible(p, shift + (r0 + rb) / g, len, lo_b, hi_b);
+        // the keys that every row of this warp sees: a tile inside them needs no mask
+        const int all_lo = __reduce_max_sync(0xffffffffu, max(lo_a, lo_b));
+        const int all_hi = __reduce_min_sync(0xffffffffu, min(ra < rows ? hi_a : 0x7fffffff, rb < rows ? hi_b : 0x7fffffff));
+        int F = -1000;                                           // frame of P: above the exponent of every V scale met so far
+        float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.0f, l_b = 0.0f;
+        float alpha_a = 0.0f, alpha_b = 0.0f;                    // weight of everything before the tile in the tile's frame
+        float2 o[32];                                            // [8 dims][row a, row b]
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = make_float2(0.f, 0.f);
+        // O of tile j: o = o * alpha + O(j)
+        auto fold = [&](int j) {
+            const int b = j & 1;
+            if (!ptx::mbar_wait(o_full(b), (j >> 1) & 1, abort_flag, p.status)) return false;
+            ptx::tc_fence_after();
+            const float2 aa = make_float2(alpha_a, alpha_a), ab = make_float2(alpha_b, alpha_b);
+#pragma unroll
+            for (int c0 = 0; c0 < PF_D; c0 += 32) {
+                uint32_t t[16];
+                ptx::tmem_ld_16x32(base + 256 + 128 * b + c0, t);
+                ptx::tmem_ld_wait();
+                if (c0 + 32 == PF_D) {
+                    ptx::tc_fence_before();
+                    ptx::mbar_arrive(o_free(b));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int k = c0 / 4 + 2 * i;
+                    o[k] = pf_fma2(o[k], aa, make_float2(__uint_as_float(t[4 * i]), __uint_as_float(t[4 * i + 1])));
+                    o[k + 1] = pf_fma2(o[k + 1], ab, make_float2(__uint_as_float(t[4 * i + 2]), __uint_as_float(t[4 * i + 3])));
+                }
+            }
+            return true;
+        };
+        bool alive = true;
+        for (int j = 0; j < n_tiles; ++j) {
+            const int b = j & 1;
+            if (!ptx::mbar_wait(par_full(j & 3), (j >> 2) & 1, abort_flag, p.status) ||
+                !ptx::mbar_wait(s_full(b), (j >> 1) & 1, abort_flag, p.status)) { alive = false; break; }
+            ptx::tc_fence_after();
+            const float* pr = par + (j & 3) * PF_PARAM_FLOATS + col;
+            const int key0 = (page_base + j * 8) * PF_BS;
+            const uint32_t s_addr = base + 128 * b;
+            uint32_t y[64];                                      // per 8 columns: row a col, col + 1, row b col, col + 1
+            ptx::tmem_ld_16x32(s_addr, y);
+            ptx::tmem_ld_16x32(s_addr + 32, y + 16);
+            ptx::tmem_ld_16x32(s_addr + 64, y + 32);
+            ptx::tmem_ld_16x32(s_addr + 96, y + 48);
+            const uint4 vmax = *reinterpret_cast<const uint4*>(pr - col + 2 * PF_KEYS), valid = *reinterpret_cast<const uint4*>(pr - col + 2 * PF_KEYS + 4);
+            ptx::tmem_ld_wait();
+            // scores in base 2
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float2 ks = *reinterpret_cast<const float2*>(pr + 8 * i);
+                const float2 a = pf_mul2(make_float2(__uint_as_float(y[4 * i]), __uint_as_float(y[4 * i + 1])), ks);
+                const float2 c = pf_mul2(make_float2(__uint_as_float(y[4 * i + 2]), __uint_as_float(y[4 * i + 3])), ks);
+                y[4 * i] = __float_as_uint(a.x); y[4 * i + 1] = __float_as_uint(a.y);
+                y[4 * i + 2] = __float_as_uint(c.x); y[4 * i + 3] = __float_as_uint(c.y);
+            }
+            if (key0 < all_lo || key0 + PF_KEYS - 1 > all_hi || (valid.x & valid.y & valid.z & valid.w) != 0xffffffffu) {
+                const uint32_t bits[4] = {valid.x, valid.y, valid.z, valid.w};
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const int c = 8 * (i >> 1) + col + (i & 1), key = key0 + c;
+                    const bool ok = (bits[i >> 3] >> (c & 31)) & 1u;
+                    if (!ok || key < lo_a || key > hi_a) y[4 * (i >> 1) + (i & 1)] = 0xff800000u;
+                    if (!ok || key < lo_b || key > hi_b) y[4 * (i >> 1) + 2 + (i & 1)] = 0xff800000u;
+                }
+            }
+            float ma[2] = {m_a, -INFINITY}, mb[2] = {m_b, -INFINITY};
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                ma[i & 1] = fmaxf(ma[i & 1], fmaxf(__uint_as_float(y[4 * i]), __uint_as_float(y[4 * i + 1])));
+                mb[i & 1] = fmaxf(mb[i & 1], fmaxf(__uint_as_float(y[4 * i + 2]), __uint_as_float(y[4 * i + 3])));
+            }
+            float na = fmaxf(ma[0], ma[1]), nb = fmaxf(mb[0], mb[1]);
+            na = fmaxf(na, __shfl_xor_sync(0xffffffffu, na, 1)); nb = fmaxf(nb, __shfl_xor_sync(0xffffffffu, nb, 1));
+            na = fmaxf(na, __shfl_xor_sync(0xffffffffu, na, 2)); nb = fmaxf(nb, __shfl_xor_sync(0xffffffffu, nb, 2));
+            const int fmax = max(PF_MIN_FRAME, static_cast<int>(max(max(vmax.x, vmax.y), max(vmax.z, vmax.w)) >> 23) - 127);
+            const int F_new = fmax > F ? fmax + 1 : F;
+            const float dF = static_cast<float>(F - F_new);
+            const float next_a = m_a == -INFINITY ? 0.0f : pf_exp2((m_a - na) + dF);     // a row without a visible key so far has nothing to keep
+            const float next_b = m_b == -INFINITY ? 0.0f : pf_exp2((m_b - nb) + dF);
+            m_a = na; m_b = nb; F = F_new;
+            const float head = static_cast<float>(PF_HEAD - F);
+            const float ea = m_a == -INFINITY ? 0.0f : head - m_a, eb = m_b == -INFINITY ? 0.0f : head - m_b;
+            const float2 ea2 = make_float2(ea, ea), eb2 = make_float2(eb, eb), minus1 = make_float2(-1.0f, -1.0f);
+            float2 la = make_float2(0.f, 0.f), lb = la;
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {                        // 16 keys: an MMA step of P
+                uint32_t w[8];                                   // columns 0-7 high halves, 8-15 low halves; rows a, b of each four
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int i = 2 * s + u;
+                    const float2 vs = *reinterpret_cast<const float2*>(pr + PF_KEYS + 8 * i);
+                    float2 a = pf_add2(make_float2(__uint_as_float(y[4 * i]), __uint_as_float(y[4 * i + 1])), ea2);
+                    float2 c = pf_add2(make_float2(__uint_as_float(y[4 * i + 2]), __uint_as_float(y[4 * i + 3])), eb2);
+                    a.x = pf_exp2(a.x); a.y = pf_exp2(a.y); c.x = pf_exp2(c.x); c.y = pf_exp2(c.y);
+                    la = pf_add2(la, a);
+                    lb = pf_add2(lb, c);
+                    a = pf_mul2(a, vs);
+                    c = pf_mul2(c, vs);
+                    const float2 ha = make_float2(pf_high(a.x), pf_high(a.y)), hc = make_float2(pf_high(c.x), pf_high(c.y));
+                    a = pf_fma2(ha, minus1, a);
+                    c = pf_fma2(hc, minus1, c);
+                    w[2 * u] = pf_pack(ha.x, ha.y);
+                    w[2 * u + 1] = pf_pack(hc.x, hc.y);
+                    w[4 + 2 * u] = pf_pack(a.x, a.y);
+                    w[4 + 2 * u + 1] = pf_pack(c.x, c.y);
+                }
+                ptx::tmem_st_16x16(s_addr + 16 * s, w);
+            }
+            ptx::tmem_st_wait();
+            ptx::tc_fence_before();
+            ptx::mbar_arrive(p_full(b));
+            l_a = fmaf(l_a, next_a, la.x + la.y);
+            l_b = fmaf(l_b, next_b, lb.x + lb.y);
+            if (j > 0 && !fold(j - 1)) { alive = false; break; }  // done long ago; this tile's PV starts meanwhile
+            alpha_a = next_a;
+            alpha_b = next_b;
+        }
+        if (alive && n_tiles > 0) alive = fold(n_tiles - 1);
+        // ---- output ----
+        if (alive) {
+            l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
+            l_a += __shfl_xor_sync(0xffffffffu, l_a, 2); l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int r = x ? rb : ra, R = r0 + r, q = R / g, h = R - q * g;
+                if (r >= rows) continue;
+                const float l = row_bad[r] ? __uint_as_float(0x7fc00000u) : x ? l_b : l_a, m = x ? m_b : m_a;
+                float f = 1.0f;
+                float* dst;
+                if (p.splits == 1) {
+                    f = (l == 0.0f) ? 0.0f : __fdiv_rn(1.0f, l);
+                    dst = p.O + ((static_cast<int64_t>(req) * p.n_q_heads + kvh * g + h) * p.seq_q + q) * PF_D;
+                } else {
+                    dst = p.part + (split * p.total_rows + (static_cast<int64_t>(req) * p.n_kv_heads + kvh) * rows_all + R) * PF_PART;
+                    // the frame of O and l: their weight against another key range's is 2^(difference)
+                    if ((lane & 3) == 0) *reinterpret_cast<float2*>(dst + PF_D) = make_float2(m == -INFINITY ? m : m + static_cast<float>(F), l);
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    *reinterpret_cast<float2*>(dst + 8 * i + col) = make_float2(o[2 * i + x].x * f, o[2 * i + x].y * f);
+            }
+        }
+    } else if (warp < 12) {
+        pf_fewer_registers<PF_REG_CONVERT>();
+        // ---- converters: warp cw owns pages 2 cw and 2 cw + 1 of every tile, thread ct the scales of token ct ----
+        const int cw = warp - 8, ct = threadIdx.x - 256;
+        const int last_page = min((len + PF_BS - 1) / PF_BS, p.max_blocks) - 1;
+        auto page_row = [&](int page) {                          // first row of a page of this head; -1: masked
+            if (page > last_page) return int64_t(-1);
+            const int blk = table[page];
+            return (blk >= 0 && blk < p.num_blocks) ? (static_cast<int64_t>(blk) * p.n_kv_heads + kvh) * PF_BS : int64_t(-1);
+        };
+        int64_t row_a = -1, row_b = -1;                          // the two pages, of the tile being loaded
+        auto load = [&](uint4 (&w)[8], const int8_t* pool) {     // 4 tokens per instruction, 512 contiguous bytes
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int64_t row = i < 4 ? row_a : row_b;
+                w[i] = row >= 0 ? __ldg(reinterpret_cast<const uint4*>(pool + row * PF_D + (i & 3) * 512 + lane * 16)) : make_uint4(0, 0, 0, 0);
+            }
+        };
+        // 16 values of token tok, d = 16 ch .. +15: half ch / 4, chunks 2 (ch % 4) and + 1, swizzled with the token;
+        // lanes of the two halves store their chunks in opposite order (no bank is met twice)
+        const int ch = lane & 7, flip = ch >> 2;
+        auto store = [&](const uint4 (&w)[8], uint8_t* tile) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int tok = cw * 32 + i * 4 + (lane >> 3);
+                uint4 a, b;
+                pf_cvt4(w[i].x, a.x, a.y); pf_cvt4(w[i].y, a.z, a.w);
+                pf_cvt4(w[i].z, b.x, b.y); pf_cvt4(w[i].w, b.z, b.w);
+                uint8_t* base = tile + flip * PF_HALF_BYTES + tok * 128;
+                const int c2 = (ch & 3) * 2;
+                *reinterpret_cast<uint4*>(base + (((c2 + flip) ^ (tok & 7)) << 4)) = flip ? b : a;
+                *reinterpret_cast<uint4*>(base + (((c2 + 1 - flip) ^ (tok & 7)) << 4)) = flip ? a : b;
+            }
+        };
+        const float s_scale = __uint_as_float(static_cast<uint32_t>(254 - q_exp) << 23) * p.scale_log2e;
+        uint4 w[8];                                              // the operand that is stored next: K(j), V(j), K(j + 1), ...
+        float ks = 0.0f, vs = 0.0f;
+        bool ok = false;
+        auto load_k = [&](int j) {
+            const int pg = page_base + j * 8 + 2 * cw;
+            row_a = page_row(pg);
+            row_b = page_row(pg + 1);
+            load(w, p.Kp);
+            const int64_t row = (lane & 16) ? row_b : row_a;     // token ct = 32 cw + lane
+            ok = row >= 0 && (page_base + j * 8) * PF_BS + ct < len;
+            if (ok) { ks = __ldg(p.Ks + row + (ct & 15)); vs = __ldg(p.Vs + row + (ct & 15)); }
+        };
+        if (n_tiles > 0) load_k(0);
+        for (int j = 0; j < n_tiles; ++j) {
+            const int b = j & 1, parity = ((j >> 1) & 1) ^ 1;
+            if (!ptx::mbar_wait(k_empty(b), parity, abort_flag, p.status)) break;
+            store(w, k_sm + b * PF_TILE_BYTES);
+            load(w, p.Vp);
+            float* pr = par + (j & 3) * PF_PARAM_FLOATS;
+            const unsigned vbits = __reduce_max_sync(0xffffffffu, ok ? __float_as_uint(vs) & 0x7fffffffu : 0u);
+            const unsigned valid = __ballot_sync(0xffffffffu, ok);
+            pr[ct] = ok ? ks * s_scale : 0.0f;
+            pr[PF_KEYS + ct] = ok ? vs : 0.0f;
+            if (lane == 0) {
+                reinterpret_cast<unsigned*>(pr)[2 * PF_KEYS + cw] = vbits;
+                reinterpret_cast<unsigned*>(pr)[2 * PF_KEYS + 4 + cw] = valid;
+            }
+            __syncwarp();
+            ptx::fence_proxy_async_smem();
+            ptx::mbar_arrive(par_full(j & 3));
+            ptx::mbar_arrive(k_full(b));
+            if (!ptx::mbar_wait(v_empty(b), parity, abort_flag, p.status)) break;
+            store(w, v_sm + b * PF_TILE_BYTES);
+            if (j + 1 < n_tiles) load_k(j + 1);
+            ptx::fence_proxy_async_smem();
+            ptx::mbar_arrive(v_full(b));
+        }
+    } else {
+        pf_fewer_registers<PF_REG_ISSUE>();
+        if (warp == 12 && ptx::elect_one()) {
+            // ---- MMA issuer ----
+            const uint32_t qa = ptx::smem_u32(q_sm), ka = ptx::smem_u32(k_sm), va = ptx::smem_u32(v_sm);
+            auto qk = [&](int j) {
+                const int b = j & 1;
+                if (!ptx::mbar_wait(k_full(b), (j >> 1) & 1, abort_flag, p.status)) return false;
+                ptx::tc_fence_after();
+#pragma unroll
+                for (int pass = 0; pass < 2; ++pass)
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        const uint32_t off = (s >> 2) * PF_HALF_BYTES + (s & 3) * 32;      // 16 of d
+                        ptx::mma_f16_ss(tmem + 128 * b, ptx::smem_desc_sw128(qa + pass * PF_TILE_BYTES + off, 16, 1024),
+                                        ptx::smem_desc_sw128(ka + b * PF_TILE_BYTES + off, 16, 1024), pf_idesc(false), (pass | s) != 0 ? 1u : 0u);
+                    }
+                ptx::tc_commit(s_full(b));
+                ptx::tc_commit(k_empty(b));
+                return true;
+            };
+            bool ok = n_tiles > 0 && qk(0);
+            if (ok && n_tiles > 1) ok = qk(1);
+            for (int j = 0; j < n_tiles && ok; ++j) {
+                const int b = j & 1, phase = (j >> 1) & 1;
+                ok = ptx::mbar_wait(v_full(b), phase, abort_flag, p.status) && ptx::mbar_wait(p_full(b), phase, abort_flag, p.status) &&
+                     ptx::mbar_wait(o_free(b), phase ^ 1, abort_flag, p.status);
+                if (!ok) break;
+                ptx::tc_fence_after();
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+#pragma unroll
+                    for (int pass = 0; pass < 2; ++pass)                                   // 16 keys of P: 8 columns
+                        ptx::mma_f16_ts(tmem + 256 + 128 * b, tmem + 128 * b + 16 * s + 8 * pass,
+                                        ptx::smem_desc_sw128(va + b * PF_TILE_BYTES + s * 2048, PF_HALF_BYTES, 1024), pf_idesc(true),
+                                        (pass | s) != 0 ? 1u : 0u);
+                ptx::tc_commit(v_empty(b));
+                ptx::tc_commit(o_full(b));
+                if (j + 2 < n_tiles) ok = qk(j + 2);              // overwrites P(j): issued after the MMAs that read it
+            }
+        }
+    }
+
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 12) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc(tmem, 512);
+    }
+}
+
+// One warp per (request, head, query): the partials of its key ranges, added in their order.
+__global__ void __launch_bounds__(256) paged_prefill_merge_kernel(const PrefillParams p) {
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (row >= p.total_rows) return;
+    float M = -INFINITY;
+    for (int s = 0; s < p.splits; ++s) M = fmaxf(M, p.part[(s * p.total_rows + row) * PF_PART + PF_D]);
+    float l = 0.0f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < p.splits; ++s) {
+        const float* src = p.part + (s * p.total_rows + row) * PF_PART;
+        const float2 ml = *reinterpret_cast<const float2*>(src + PF_D);
+        if (ml.x == -INFINITY && ml.y == 0.0f) continue;         // this range saw no key
+        const float f = ml.x == -INFINITY ? 1.0f : pf_exp2(ml.x - M);   // without a key but l = NaN: a non-finite row stays so
+        const float2 a = *reinterpret_cast<const float2*>(src + 4 * lane), b = *reinterpret_cast<const float2*>(src + 4 * lane + 2);
+        l = fmaf(f, ml.y, l);
+        o.x = fmaf(f, a.x, o.x); o.y = fmaf(f, a.y, o.y); o.z = fmaf(f, b.x, o.z); o.w = fmaf(f, b.y, o.w);
+    }
+    const float inv = (l == 0.0f) ? 0.0f : __fdiv_rn(1.0f, l);
+    const int rows_all = p.seq_q * p.group;
+    const int64_t rk = row / rows_all;                           // req * n_kv_heads + kv head
+    const int R = static_cast<int>(row - rk * rows_all), q = R / p.group, h = R - q * p.group;
+    const int64_t req = rk / p.n_kv_heads, kvh = rk - req * p.n_kv_heads;
+    float* dst = p.O + ((req * p.n_q_heads + kvh * p.group + h) * p.seq_q + q) * PF_D + 4 * lane;
+    *reinterpret_cast<float4*>(dst) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+}
+
+bool prefill_fast_ok(const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L) {
+    return cfg.seq_q > 1 && cfg.head_dim == PF_D && L.head_dim == PF_D && L.block_size == PF_BS && cfg.n_kv_heads > 0 &&
+           cfg.n_kv_heads <= 65535 && cfg.n_q_heads % cfg.n_kv_heads == 0 &&
+           static_cast<int64_t>(cfg.seq_q) * (cfg.n_q_heads / cfg.n_kv_heads) < (int64_t(1) << 30);
+}
+
+int launch_prefill_fast(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int8_t* Vp, const float* Ks, const float* Vs,
+                        const int32_t* tables, int max_blocks, const int32_t* seq_lens, int seq_len_scalar, int n_req,
+                        float* O, const lhb_paged_attn_cfg& cfg, const lhb_paged_layout& L, cudaStream_t st) {
+    PrefillParams p{};
+    p.Q = Q; p.Kp = Kp; p.Vp = Vp; p.Ks = Ks; p.Vs = Vs; p.tables = tables; p.seq_lens = seq_lens; p.O = O;
+    p.status = ctx->status_word;
+    p.seq_len_scalar = seq_len_scalar; p.max_blocks = max_blocks; p.num_blocks = L.num_blocks;
+    p.n_q_heads = cfg.n_q_heads; p.n_kv_heads = cfg.n_kv_heads; p.group = cfg.n_q_heads / cfg.n_kv_heads; p.seq_q = cfg.seq_q;
+    p.causal = cfg.causal; p.window = cfg.window; p.chunk = cfg.chunk;
+    const int rows = p.seq_q * p.group;
+    p.row_tiles = ceil_div(rows, PF_ROWS);
+    p.total_rows = static_cast<int64_t>(n_req) * p.n_kv_heads * rows;
+    const float scale = cfg.scale > 0.0f ? cfg.scale : 1.0f / sqrtf(static_cast<float>(cfg.head_dim));
+    p.scale_log2e = scale * 1.4426950408889634f;
+    p.part = reinterpret_cast<float*>(ctx->scratch);
+    // Key splits: the longest request's tiles against the waves of CTAs.  A CTA spends about two tiles' time on
+    // set-up and output; a split costs the merge launch besides (about two more).
+    int64_t keys = seq_lens ? static_cast<int64_t>(max_blocks) * PF_BS : seq_len_scalar;
+    if (p.window > 0) keys = std::min<int64_t>(keys, static_cast<int64_t>(p.window) + PF_ROWS / p.group + 1);
+    const int64_t tiles = std::max<int64_t>(1, (keys + PF_KEYS - 1) / PF_KEYS);
+    const int64_t ctas = static_cast<int64_t>(p.row_tiles) * p.n_kv_heads * n_req;
+    int64_t best = -1;
+    p.splits = 1;
+    for (int s = 1; s <= 32 && s <= tiles; ++s) {
+        if (s > 1 && static_cast<size_t>(s) * p.total_rows * PF_PART * sizeof(float) > ctx->scratch_bytes) break;
+        const int64_t waves = (ctas * s + ctx->sm_count - 1) / ctx->sm_count;
+        const int64_t cost = waves * ((tiles + s - 1) / s + 2) + (s > 1 ? 2 : 0);
+        if (best < 0 || cost < best) { best = cost; p.splits = s; }
+    }
+    if (static_cast<int64_t>(p.row_tiles) * p.splits > (int64_t(1) << 30)) return LHB_ERR_UNSUPPORTED;
+    static bool attr_set[64] = {};
+    if (!attr_set[ctx->device & 63]) {
+        LHB_CUDA(cudaFuncSetAttribute(paged_prefill_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PF_SMEM)));
+        attr_set[ctx->device & 63] = true;
+    }
+    paged_prefill_q8_kernel<<<dim3(p.row_tiles * p.splits, p.n_kv_heads, n_req), PF_THREADS, PF_SMEM, st>>>(p);
+    LHB_LAUNCH_CHECK();
+    if (p.splits > 1) {
+        paged_prefill_merge_kernel<<<static_cast<unsigned>(ceil_div64(p.total_rows, 8)), 256, 0, st>>>(p);
+        LHB_LAUNCH_CHECK();
+    }
+    return LHB_OK;
+}
+
+}  // namespace lhb

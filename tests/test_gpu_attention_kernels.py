@@ -68,3 +68,55 @@ def test_decode_attention_fp32_pools(chk, qh, kvh, window, chunk, lens):
         got = lb.paged_attention_batched_f32(dev(Q), dev(kp), dev(vp), dev(holed), dev(sl), lb_cfg(cfg), lb_layout(L))
         assert np.isfinite(host(got)).all()
     poll_ok()
+
+
+@pytest.mark.parametrize("seq_q,lens,qh,kvh,causal,window,chunk", [
+    (2, [2, 1, 0], 4, 1, 1, 0, 0),            # a request shorter than its query rows, an empty one
+    (32, [32], 4, 1, 1, 0, 0),                # one full row tile, page-aligned keys
+    (33, [161, 128, 129], 8, 2, 1, 0, 0),     # a second row tile of four rows; key tiles full, one over
+    (65, [700], 4, 1, 1, 0, 0),               # two CTAs of rows, keys split over CTAs
+    (3, [2050], 8, 8, 1, 0, 0),               # few rows, many keys: many key ranges, one head per KV head
+    (50, [300, 75], 6, 2, 1, 40, 0),          # group of three, sliding window
+    (70, [513], 16, 2, 1, 0, 96),             # group of eight, chunked mask
+    (20, [150], 4, 2, 0, 0, 0),               # not causal
+    (20, [150, 9], 4, 2, 0, 30, 64),          # window and chunk without causality
+])
+def test_prefill_attention(chk, seq_q, lens, qh, kvh, causal, window, chunk):
+    rng = np.random.default_rng(seq_q + sum(lens))
+    L, tables, pools, (k, v, ks, vs) = build_paged_case(chk, rng, len(lens), lens, qh, kvh, 128, 16, blocks(lens))
+    cfg = AttnCfg(qh, kvh, seq_q, 128, causal, 0.0, window, chunk)
+    Q = (rng.standard_normal((len(lens), qh, seq_q, 128)) * rng.choice([0.01, 1.0, 3.0], size=(1, qh, 1, 1))).astype(np.float32)
+    sl = np.array(lens, np.int32)
+    want = chk.paged_attention_q8_batched(Q, pools, tables, sl, cfg, L, parallel=True)
+    got = lb.paged_attention_q8_batched(dev(Q), k, v, ks, vs, dev(tables), dev(sl), lb_cfg(cfg), lb_layout(L))
+    assert_close(host(got), want, what="prefill, batched call")
+    for r, n in enumerate(lens):
+        one = lb.paged_attention_q8(dev(Q[r]), k, v, ks, vs, dev(tables[r]), n, lb_cfg(cfg), lb_layout(L))
+        assert_close(host(one), want[r], what=f"prefill, request {r} alone")
+    poll_ok()
+
+
+def test_prefill_attention_holes_and_row_scales(chk):
+    """A table entry outside the pool masks its 16 keys; V rows whose scales differ by 2^20 and rows of rising
+    scores (the running maximum moves in every key tile) keep their precision: fp64 softmax over the remaining keys."""
+    rng = np.random.default_rng(5)
+    seq_q, n, qh, kvh = 40, 600, 4, 2
+    L, tables, pools, (k, v, ks, vs) = build_paged_case(chk, rng, 1, [n], qh, kvh, 128, 16, blocks([n]))
+    vs *= torch.exp2(torch.randint(-10, 11, vs.shape, device="cuda").float())
+    ks *= torch.linspace(0.5, 4.0, ks.numel(), device="cuda").view(ks.shape)
+    holed = tables.copy()
+    holed[0, 3], holed[0, 20] = -1, L.num_blocks + 7
+    Q = (2.0 * rng.standard_normal((1, qh, seq_q, 128))).astype(np.float32)
+    cfg = AttnCfg(qh, kvh, seq_q, 128, 1, 0.0, 0, 0)
+    got = host(lb.paged_attention_q8_batched(dev(Q), k, v, ks, vs, dev(holed), dev(np.array([n], np.int32)), lb_cfg(cfg), lb_layout(L)))
+    kd, vd = host(k).astype(np.float64) * host(ks)[..., None], host(v).astype(np.float64) * host(vs)[..., None]
+    for h in range(qh):
+        for i in range(seq_q):
+            keys = np.array([j for j in range(n - seq_q + i + 1) if 0 <= holed[0, j // 16] < L.num_blocks])
+            blk, slot = holed[0, keys // 16], keys % 16
+            s = kd[blk, h // 2, slot] @ Q[0, h, i].astype(np.float64) / np.sqrt(128)
+            w = np.exp(s - s.max()); w /= w.sum()
+            want = w @ vd[blk, h // 2, slot]
+            scale = max(1.0, np.abs(want).max())               # the absolute term is stated for values of order one
+            assert_close(got[0, h, i] / scale, want / scale, what=f"head {h} row {i}")
+    poll_ok()
