@@ -20,7 +20,7 @@ OBJ = os.path.join(PKG, "_obj")
 LIB = os.path.join(PKG, "lib", "liblhb200.so")
 
 SOURCES = ["api.cu", "quant.cu", "gemm_generic.cu", "kvcache.cu", "paged_attention_generic.cu",
-           "tensor_map.cu", "gemv_mma.cu", "gemm_w4a16_tc.cu", "gemm_w8a8_tc.cu", "paged_attention_decode.cu",
+           "tensor_map.cu", "gemv_mma.cu", "gemm_w4a16_tc.cu", "gemm_wo_wide.cu", "gemm_w8a8_tc.cu", "paged_attention_decode.cu",
            "paged_attention_decode_f32.cu", "paged_attention_prefill.cu",
            "cache_manager.cu", "glue.cu", "quant_asym.cu", "fp8.cu", "peer_gather.cu", "peer_vmm.cu", "lh_dropin.cu"]
 

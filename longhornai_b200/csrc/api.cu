@@ -115,6 +115,10 @@ int lhb_gemm_w4a16_groupwise(lhb_ctx* ctx, const float* A, const uint8_t* Bp, co
     if (M == 0) return LHB_OK;
     cudaStream_t st = as_stream(stream);
     const bool al = aligned16(A) && aligned16(Bp) && aligned16(Bs) && aligned16(C);
+    if (al && wo_wide_prefer(0, M, N, K, G)) {
+        const int e = launch_wo_wide(ctx, 0, A, Bp, Bs, nullptr, C, M, N, K, G, alpha, beta, st);
+        if (e != LHB_ERR_UNSUPPORTED) return e;              // an arena too small for its halves: the slab kernels
+    }
     if (al && M >= w4a16_tc_min_rows() && w4a16_tc_ok(M, N, K, G))
         return launch_w4a16_tc(ctx, A, Bp, Bs, C, M, N, K, G, alpha, beta, st, 0, nullptr, 0.0f);
     if (w4a16_fast_ok(M, N, K, G) && al)
@@ -153,7 +157,12 @@ int lhb_gemm_w8a16_perchannel(lhb_ctx* ctx, const float* A, const int8_t* Bq, co
     if (M < 0 || N <= 0 || K <= 0) return LHB_ERR_BAD_SHAPE;
     if (M == 0) return LHB_OK;
     cudaStream_t st = as_stream(stream);
-    if (w8a16_fast_ok(M, N, K) && aligned16(A) && aligned16(Bq) && aligned16(Bs) && aligned16(C))
+    const bool al = aligned16(A) && aligned16(Bq) && aligned16(Bs) && aligned16(C);
+    if (al && wo_wide_prefer(2, M, N, K, 0)) {
+        const int e = launch_wo_wide(ctx, 2, A, Bq, Bs, nullptr, C, M, N, K, 0, alpha, beta, st);
+        if (e != LHB_ERR_UNSUPPORTED) return e;
+    }
+    if (w8a16_fast_ok(M, N, K) && al)
         return launch_w8a16_fast(ctx, A, Bq, Bs, C, M, N, K, alpha, beta, st);
     return launch_w8a16_generic(A, Bq, Bs, C, M, N, K, alpha, beta, st);
 }
@@ -166,12 +175,15 @@ int lhb_gemm_w4a16_groupwise_prologue(lhb_ctx* ctx, const float* X, int prologue
     if (prologue == 1 && !gamma) return LHB_ERR_NULL;
     if (M < 0 || N <= 0 || K <= 0 || G <= 0 || (K % 2) || (K % G)) return LHB_ERR_BAD_SHAPE;
     if (M == 0) return LHB_OK;
-    if (M >= w4a16_tc_min_rows() && w4a16_tc_ok(M, N, K, G) && aligned16(X) && aligned16(Bp) && aligned16(Bs) &&
-        aligned16(C) && (prologue != 1 || aligned16(gamma)))
+    const bool al = aligned16(X) && aligned16(Bp) && aligned16(Bs) && aligned16(C) && (prologue != 1 || aligned16(gamma));
+    if (al && wo_wide_prefer(0, M, N, K, G)) {
+        const int e = launch_wo_wide(ctx, 0, X, Bp, Bs, nullptr, C, M, N, K, G, alpha, beta, as_stream(stream), prologue, gamma, eps);
+        if (e != LHB_ERR_UNSUPPORTED) return e;
+    }
+    if (M >= w4a16_tc_min_rows() && w4a16_tc_ok(M, N, K, G) && al)
         return launch_w4a16_tc(ctx, X, Bp, Bs, C, M, N, K, G, alpha, beta, as_stream(stream), prologue, gamma, eps);
     if (M - ((M - 1) / 16) * 16 <= 2) return LHB_ERR_UNSUPPORTED;   // a last slab of one or two rows has no digit pass
-    if (!(w4a16_fast_ok(M, N, K, G) && aligned16(X) && aligned16(Bp) && aligned16(Bs) && aligned16(C) &&
-          (prologue != 1 || aligned16(gamma))))
+    if (!(w4a16_fast_ok(M, N, K, G) && al))
         return LHB_ERR_UNSUPPORTED;       // the caller runs lhb_rmsnorm / lhb_swiglu and the plain GEMM instead
     return launch_w4a16_fast_prologue(ctx, X, prologue, gamma, eps, Bp, Bs, C, M, N, K, G, alpha, beta,
                                       as_stream(stream));

@@ -97,6 +97,14 @@ bool w4a16_asym_fast_ok(int M, int N, int K, int G);
 int launch_w4a16_asym_fast(lhb_ctx* ctx, const float* A, const uint8_t* Bp, const uint16_t* Bs, const uint16_t* Bz,
                            float* C, int M, int N, int K, int G, float alpha, float beta, cudaStream_t st);
 
+// weight-only GEMMs with many rows, tcgen05 (gemm_wo_wide.cu).  fmt 0: int4 groups (scales fp32 [K/G, N]), 1: asymmetric int4
+// (scales and zeros fp16 [K/G, N]), 2: int8 per channel (scales fp32 [N]).  wo_wide_prefer: whether M rows are many enough.
+bool wo_wide_ok(int fmt, int M, int N, int K, int G);
+bool wo_wide_prefer(int fmt, int M, int N, int K, int G);
+int launch_wo_wide(lhb_ctx* ctx, int fmt, const float* A, const void* B, const void* scales, const void* zeros, float* C, int M,
+                   int N, int K, int G, float alpha, float beta, cudaStream_t st, int prologue = 0,
+                   const float* gamma = nullptr, float eps = 0.0f);
+
 // TMA tensor maps (tensor_map.cu): 2-D uint8 tensor [rows, cols] (cols
 // contiguous, row pitch in bytes), box [box_rows, box_cols], 128-byte swizzle
 // when swizzle128 is set.  Cached per context.
@@ -109,6 +117,8 @@ int get_tensor_map_2d_f32(lhb_ctx* ctx, const void* base, uint64_t rows, uint64_
                           uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols, TensorMap* out);
 // fp32 with the 128-byte swizzle (box_cols * 4 == 128): the target of bulk stores from swizzled staging tiles
 int get_tensor_map_2d_f32_sw128(lhb_ctx* ctx, const void* base, uint64_t rows, uint64_t cols,
+                                uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols, TensorMap* out);
+int get_tensor_map_2d_f16_sw128(lhb_ctx* ctx, const void* base, uint64_t rows, uint64_t cols,
                                 uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols, TensorMap* out);
 // and for an fp16 tensor
 int get_tensor_map_2d_f16(lhb_ctx* ctx, const void* base, uint64_t rows, uint64_t cols,

@@ -1,0 +1,630 @@
+// Weight-only GEMMs with many activation rows (prefill) on the 5th-generation tensor cores: int4 group-wise
+// (src/kernels/gemm_quant.cpp:54-82), asymmetric int4 and int8 per channel, weights in their storage layout.
+//
+//   C[m][n] = beta C + alpha * sum_g s[g][n] * sum_{k in g} A[m][k] w[k][n],    A fp32, w small integers
+//
+// Integers up to 11 bits are exact in fp16, so the inner sums run as two kind::f16 passes: every activation row
+// is scaled by a power of two (wide_digits_kernel, with RMSNorm or SwiGLU on the way where asked) and split into
+// a high and a low fp16 of 11 bits each.  Both passes add to one fp32 accumulator per quantisation group (at
+// most 128 k: 16 steps, the low halves of a chunk first, so that the truncating additions of the tensor
+// core stay at the level of one fp32 rounding), and the group sums are scaled and added in fp32 registers.
+//
+// A CTA pair owns 256 weight columns x up to 256 rows.  The weights are the 128-lane operand (128 columns per
+// CTA), so that a column's group scale is one register of its epilogue thread; the activation rows are the
+// other operand, half of them fetched by each CTA.  Roles (512 threads a CTA):
+//   warps 0-7    epilogue: column = TMEM lane, warps 0-3 the first half of the rows, 4-7 the second, up to 128 fp32
+//                sums a thread; accumulators double-buffered in the 512 TMEM columns
+//   warps 8-11   converters: packed bytes -> registers (three chunks ahead) -> fp16 -> 128-byte-swizzled tile.  A
+//                nibble under the exponent byte 0x64 is 1024 + u; the high nibble needs no shift (1024 + 16 u, one
+//                fused multiply-add); an asymmetric weight subtracts its zero-point instead of the constant
+//   warp 12      TMA producer of the activation tiles, warp 13 MMA issuer (in the leader), warp 14 TMEM
+// What bounds it: per k a pair spends 16 tensor cycles on 256 x 256; the shared memory of each CTA moves 120 bytes
+// a cycle for that (operand reads 1024 B, tile fills 896 B per k).  A single CTA on 128 x 256 would need 184
+// of its 128 bytes a cycle: hence the pair.  The rows per tile (a multiple of 32) are chosen so that the tiles
+// fill whole waves of pairs; where there are too few tiles, K is split over pairs and a second kernel adds
+// the parts in order.
+//
+// Every wait is bounded (ptx::mbar_wait): a timeout sets the context's status word, the roles fall
+// through to the common exit and TMEM is freed.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "dispatch.h"
+#include "ptx.cuh"
+
+namespace lhb {
+
+constexpr int WW_COLS = 256;                        // weight columns of a pair
+constexpr int WW_MAX_ROWS = 256;                    // activation rows of a tile
+constexpr int WW_CHUNK = 64;                        // k of a stage
+constexpr int WW_STAGES = 4;
+constexpr int WW_A_BYTES = 128 * WW_CHUNK * 2;      // this CTA's 128 columns, fp16: two 64-column halves
+constexpr int WW_B_BYTES = 128 * WW_CHUNK * 2;      // up to 128 rows of the high (or low) halves
+constexpr int WW_STAGE_BYTES = WW_A_BYTES + 2 * WW_B_BYTES;
+constexpr int WW_THREADS = 512;
+constexpr size_t WW_SMEM = 1024 + size_t(WW_STAGES) * WW_STAGE_BYTES + 256;
+// Registers a thread after the split; the sum is what the launch allocates (4 x 128)
+constexpr int WW_REG_EPI = 184, WW_REG_CONV = 96, WW_REG_REST = 40;
+static_assert(2 * WW_REG_EPI + WW_REG_CONV + WW_REG_REST <= 4 * 128, "register split exceeds the launch");
+
+enum { WW_W4 = 0, WW_W4A = 1, WW_W8 = 2 };
+
+struct WideParams {
+    const uint8_t* B;           // W4: packed [K/2, N]; W8: int8 [K, N]
+    const void* scales;         // W4: fp32 [K/G, N]; W4A: fp16 [K/G, N]; W8: fp32 [N]
+    const uint16_t* zeros;      // W4A: fp16 [K/G, N]
+    float* C;                   // [M, N]
+    float* part;                // [splits][M][N] when K is split
+    const float* inv_scale;     // [M]
+    int M, N, K, G;
+    int unit;                   // k of an accumulator: min(G, 128) (W8: 128, the last one may be 64)
+    int rows;                   // rows of a tile, a multiple of 32
+    int m_blocks, col_tiles, splits;
+    float alpha, beta;
+    int* status;
+};
+
+// fp16 x fp16 -> f32 (bits 4-5 = 1), A = weights MN-major (bit 15), B = activations K-major, N >> 3 at bit 17, M = 256
+__device__ __forceinline__ uint32_t ww_idesc(int n) {
+    return (1u << 4) | (1u << 15) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
+}
+
+// ---- activation halves ------------------------------------------------------------------
+// One CTA per row: optional RMSNorm (gamma, eps) or SwiGLU of a [gate || value] row, a power of two taking the
+// row's largest magnitude into [2^14, 2^15), high and low fp16 halves.
+__global__ void __launch_bounds__(512)
+wide_digits_kernel(const float* __restrict__ A, int K, __half* __restrict__ hi, __half* __restrict__ lo,
+                   float* __restrict__ inv_scale, int prologue, const float* __restrict__ gamma, float eps) {
+    __shared__ unsigned s_max[16];
+    __shared__ float s_sum[16];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // A comes from the kernel before; so may readers of hi and lo
+    const int64_t r = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* row = A + r * (prologue == 2 ? 2 * static_cast<int64_t>(K) : K);
+    constexpr int DC = 8;                                   // float4s a thread keeps; longer rows are read again
+    const bool cached = K <= 2048 * DC;
+    float4 v[DC];
+    float inv_rms = 1.0f;
+    auto raw = [&](int k) { return *reinterpret_cast<const float4*>(row + k); };
+    if (cached) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) {
+            const int k = threadIdx.x * 4 + i * 2048;
+            v[i] = k < K ? raw(k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    if (prologue == 1) {
+        float ss = 0.0f;
+        auto add = [&](float4 x) { ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w; };
+        if (cached) {
+#pragma unroll
+            for (int i = 0; i < DC; ++i) add(v[i]);
+        } else {
+            for (int k = threadIdx.x * 4; k < K; k += 2048) add(raw(k));
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) s_sum[warp] = ss;
+        __syncthreads();
+        ss = s_sum[0];
+#pragma unroll
+        for (int w = 1; w < 16; ++w) ss += s_sum[w];        // same order in every thread
+        inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, static_cast<float>(K)), eps)));
+    }
+    auto transform = [&](float4 x, int k) {
+        if (prologue == 1) {
+            const float4 g = *reinterpret_cast<const float4*>(gamma + k);
+            x.x = __fmul_rn(__fmul_rn(x.x, inv_rms), g.x); x.y = __fmul_rn(__fmul_rn(x.y, inv_rms), g.y);
+            x.z = __fmul_rn(__fmul_rn(x.z, inv_rms), g.z); x.w = __fmul_rn(__fmul_rn(x.w, inv_rms), g.w);
+        } else if (prologue == 2) {
+            const float4 u = *reinterpret_cast<const float4*>(row + K + k);
+            x.x = swiglu_one(x.x, u.x); x.y = swiglu_one(x.y, u.y); x.z = swiglu_one(x.z, u.z); x.w = swiglu_one(x.w, u.w);
+        }
+        return x;
+    };
+    unsigned mb = 0u;                                       // largest magnitude as bits: NaN and Inf survive the maximum
+    if (cached) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) {
+            const int k = threadIdx.x * 4 + i * 2048;
+            if (k < K) v[i] = transform(v[i], k);
+            mb = max(mb, abs_bits_max4(v[i]));
+        }
+    } else {
+        for (int k = threadIdx.x * 4; k < K; k += 2048) mb = max(mb, abs_bits_max4(transform(raw(k), k)));
+    }
+    mb = __reduce_max_sync(0xffffffffu, mb);
+    if (lane == 0) s_max[warp] = mb;
+    __syncthreads();
+    mb = s_max[0];
+#pragma unroll
+    for (int w = 1; w < 16; ++w) mb = max(mb, s_max[w]);
+    int se = mb ? 268 - static_cast<int>((mb >> 23) & 0xff) : 127;
+    se = max(1, min(253, se));
+    const float scl = mb >= 0x7f800000u ? 0.0f : __uint_as_float(static_cast<uint32_t>(se) << 23);
+    if (threadIdx.x == 0) inv_scale[r] = digit_inv_scale(mb, se);        // NaN for a non-finite row
+    auto put = [&](int k, float4 x) {
+        if (scl == 0.0f) x = make_float4(0.f, 0.f, 0.f, 0.f);
+        x.x *= scl; x.y *= scl; x.z *= scl; x.w *= scl;
+        const float hx = ptx::f16_high(x.x), hy = ptx::f16_high(x.y), hz = ptx::f16_high(x.z), hw = ptx::f16_high(x.w);
+        *reinterpret_cast<uint2*>(hi + r * K + k) = make_uint2(ptx::pack_f16(hx, hy), ptx::pack_f16(hz, hw));
+        *reinterpret_cast<uint2*>(lo + r * K + k) = make_uint2(ptx::pack_f16(x.x - hx, x.y - hy), ptx::pack_f16(x.z - hz, x.w - hw));
+    };
+    if (cached) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) {
+            const int k = threadIdx.x * 4 + i * 2048;
+            if (k < K) put(k, v[i]);
+        }
+    } else {
+        for (int k = threadIdx.x * 4; k < K; k += 2048) put(k, transform(raw(k), k));
+    }
+}
+
+// ---- weights to fp16 ----------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t ww_hsub2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t ww_hfma2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+// Four bytes of one k pair -> the weights of the even k (low nibbles) and of the odd k (high nibbles), two columns a word.
+// `bias` of columns (0, 1) and (2, 3): 1024 + 8 for two's complement nibbles (u = q ^ 8), 1024 + z for unsigned ones.
+template <bool ASYM>
+__device__ __forceinline__ void ww_nibbles(uint32_t w, uint32_t bias01, uint32_t bias23, uint32_t (&even)[2], uint32_t (&odd)[2]) {
+    if (!ASYM) w ^= 0x88888888u;
+    const uint32_t l = w & 0x0f0f0f0fu, h = w & 0xf0f0f0f0u;
+    even[0] = ww_hsub2(__byte_perm(l, 0x64646464u, 0x4140), bias01);
+    even[1] = ww_hsub2(__byte_perm(l, 0x64646464u, 0x4342), bias23);
+    // 1024 + 16 u: times 1/16 plus 960 - bias, exact
+    const uint32_t sixteenth = 0x2c002c00u;
+    const uint32_t n01 = ASYM ? ww_hsub2(0x63806380u, bias01) : 0xd480d480u /* -72 */, n23 = ASYM ? ww_hsub2(0x63806380u, bias23) : 0xd480d480u;
+    odd[0] = ww_hfma2(__byte_perm(h, 0x64646464u, 0x4140), sixteenth, n01);
+    odd[1] = ww_hfma2(__byte_perm(h, 0x64646464u, 0x4342), sixteenth, n23);
+}
+
+// ---- the GEMM -----------------------------------------------------------------------------
+
+template <int FMT>
+__global__ void __launch_bounds__(WW_THREADS, 1)
+gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constant__ TensorMap tmLo, const WideParams p) {
+    extern __shared__ uint8_t ww_smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ww_smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WW_STAGES * WW_STAGE_BYTES);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * WW_STAGES + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
+    const uint32_t rank = ptx::cluster_ctarank();            // 0 = leader
+    const uint32_t bar0 = ptx::smem_u32(bars);
+    auto a_full = [&](int s) { return bar0 + 8 * s; };                           // leader: both CTAs' weight tiles are stored
+    auto b_full = [&](int s) { return bar0 + 8 * (WW_STAGES + s); };             // leader: both CTAs' activation tiles have landed
+    auto empty = [&](int s) { return bar0 + 8 * (2 * WW_STAGES + s); };          // each CTA: the stage has been multiplied
+    auto t_full = [&](int b) { return bar0 + 8 * (3 * WW_STAGES + b); };         // each CTA: an accumulator is complete
+    auto t_empty = [&](int b) { return bar0 + 8 * (3 * WW_STAGES + 2 + b); };    // leader: both CTAs have read it
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < WW_STAGES; ++s) {
+            ptx::mbar_init(a_full(s), 8);
+            ptx::mbar_init(b_full(s), 1);
+            ptx::mbar_init(empty(s), 1);
+        }
+        for (int b = 0; b < 2; ++b) { ptx::mbar_init(t_full(b), 1); ptx::mbar_init(t_empty(b), 16); }
+        *abort_flag = 0;
+        ptx::fence_mbar_init();
+        ptx::prefetch_tmap(&tmHi);
+        ptx::prefetch_tmap(&tmLo);
+    }
+    if (warp == 14) {
+        ptx::tmem_alloc_pair(ptx::smem_u32(tmem_slot), 512);
+        ptx::tmem_relinquish_pair();
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::cluster_sync_all();                                 // both CTAs' barriers exist before anyone signals them
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int tiles = p.m_blocks * p.col_tiles, items = tiles * p.splits;
+    const int k_blocks = (p.K + 127) / 128;
+    // item -> rows m0 .., columns n0 .. of this CTA, k range; row blocks run fastest: neighbouring pairs share weights in L2
+    auto item_m = [&](int it) { return (it % tiles) % p.m_blocks * p.rows; };
+    auto item_n = [&](int it) { return (it % tiles) / p.m_blocks * WW_COLS + 128 * static_cast<int>(rank); };
+    auto item_k0 = [&](int it) { return static_cast<int>(static_cast<int64_t>(k_blocks) * (it / tiles) / p.splits) * 128; };
+    auto item_k1 = [&](int it) { return min(p.K, static_cast<int>(static_cast<int64_t>(k_blocks) * (it / tiles + 1) / p.splits) * 128); };
+
+    if (warp < 8) {
+        ptx::more_registers<WW_REG_EPI>();
+        // ---- epilogue ----
+        const int half = warp >> 2, cl = 32 * (warp & 3) + lane;          // which rows of the tile; column = TMEM lane
+        const int hrows = p.rows / 2;                                     // a multiple of 16
+        const uint32_t d_base = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + half * hrows;
+        uint32_t done = 0;                                                // accumulators read so far
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        bool alive = true;
+        for (int it = pair; it < items && alive; it += n_pairs) {
+            const int m0 = item_m(it) + half * hrows, n = item_n(it) + cl, k0 = item_k0(it), k1 = item_k1(it);
+            const bool col_ok = n < p.N;
+            float2 acc[64];
+#pragma unroll
+            for (int i = 0; i < 64; ++i) acc[i] = make_float2(0.f, 0.f);
+            auto scale_of = [&](int k) {
+                if (FMT == WW_W8) return 1.0f;
+                if (!col_ok || k >= k1) return 0.0f;
+                const int64_t i = static_cast<int64_t>(k / p.G) * p.N + n;
+                return FMT == WW_W4 ? __ldg(static_cast<const float*>(p.scales) + i)
+                                    : __half2float(__ushort_as_half(__ldg(static_cast<const uint16_t*>(p.scales) + i)));
+            };
+            float s_next = scale_of(k0), s_next2 = scale_of(k0 + p.unit);  // two accumulators ahead
+            for (int k = k0; k < k1; k += p.unit, ++done) {
+                const float s = s_next;
+                s_next = s_next2;
+                s_next2 = scale_of(k + 2 * p.unit);
+                const int b = done & 1;
+                if (!ptx::mbar_wait(t_full(b), (done >> 1) & 1, abort_flag, p.status)) { alive = false; break; }
+                ptx::tc_fence_after();
+                const float2 s2 = make_float2(s, s);
+                const uint32_t d_addr = d_base + 256 * b;
+                uint32_t d[2][16];
+                ptx::tmem_ld_32x16(d_addr, d[0]);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    if (16 * c < hrows) {
+                        ptx::tmem_ld_wait();
+                        if (16 * (c + 1) < hrows) {
+                            if (c < 7) ptx::tmem_ld_32x16(d_addr + 16 * (c + 1), d[(c + 1) & 1]);
+                        } else {                                          // the last columns are here: the accumulator may be overwritten
+                            ptx::tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(t_empty(b), 0));
+                        }
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            acc[8 * c + i] = ptx::fma2(make_float2(__uint_as_float(d[c & 1][2 * i]), __uint_as_float(d[c & 1][2 * i + 1])), s2, acc[8 * c + i]);
+                    }
+                }
+            }
+            if (!alive) break;
+            if (col_ok) {
+            const float cs = FMT == WW_W8 ? __ldg(static_cast<const float*>(p.scales) + n) : 1.0f;
+            float* out = p.splits > 1 ? p.part + static_cast<int64_t>(it / tiles) * p.M * p.N : p.C;
+            // eight rows at a time: their factors (and old values) are read together
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                if (8 * c < hrows && m0 + 8 * c < p.M) {
+                    float inv[8], old[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int m = min(m0 + 8 * c + i, p.M - 1);
+                        inv[i] = __ldg(p.inv_scale + m);
+                        old[i] = (p.splits == 1 && p.beta != 0.0f) ? out[static_cast<int64_t>(m) * p.N + n] : 0.0f;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int m = m0 + 8 * c + i;
+                        const float v = cs * (inv[i] * ((i & 1) ? acc[4 * c + i / 2].y : acc[4 * c + i / 2].x));
+                        if (m < p.M)
+                            out[static_cast<int64_t>(m) * p.N + n] = p.splits > 1 ? v : p.beta == 0.0f ? p.alpha * v : fmaf(p.beta, old[i], p.alpha * v);
+                    }
+                }
+            }
+            }
+            __syncwarp();
+        }
+    } else if (warp < 12) {
+        ptx::fewer_registers<WW_REG_CONV>();
+        // ---- converters: 16 columns x (W4: 2 k pairs, W8: 4 k) a thread and chunk ----
+        const int ct = threadIdx.x - 256, ch = ct & 7, kr = ct >> 3;      // 16-column chunk of the 128, row of 16
+        constexpr int LOADS = FMT == WW_W8 ? 4 : 2;                       // rows kr, kr + 16, ... of the chunk's 64 k or 32 k pairs
+        // chunks run on across items: (item, k) of the chunk being loaded
+        int l_it = pair, l_k = pair < items ? item_k0(pair) : 0, l_k1 = pair < items ? item_k1(pair) : 0;
+        auto load = [&](uint4 (&w)[LOADS]) {
+            if (l_it >= items) return;
+            const int n = item_n(l_it) + 16 * ch;
+#pragma unroll
+            for (int i = 0; i < LOADS; ++i) {
+                const int row = (FMT == WW_W8 ? l_k : l_k / 2) + kr + 16 * i;
+                const bool ok = n < p.N && (FMT == WW_W8 ? row : 2 * row) < l_k1;                    // N % 16 == 0
+                w[i] = ok ? __ldg(reinterpret_cast<const uint4*>(p.B + static_cast<int64_t>(row) * p.N + n)) : make_uint4(0, 0, 0, 0);
+            }
+            l_k += WW_CHUNK;
+            if (l_k >= l_k1) {
+                l_it += n_pairs;
+                if (l_it < items) { l_k = item_k0(l_it); l_k1 = item_k1(l_it); }
+            }
+        };
+        uint4 w[3][LOADS];                                                // the set of chunk c is c % 3: three chunks ahead
+        load(w[0]);
+        load(w[1]);
+        load(w[2]);
+        uint32_t bias[8];                                                 // per column pair; W4A: of the current group
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bias[i] = 0x64086408u;                // 1032
+        // 16 columns of row kk: two 16-byte chunks of the 64-column half, swizzled with kk % 8.  Lanes of the two
+        // halves (same banks) store their chunks in opposite order.
+        const int flip = ch >> 2, c2 = (ch & 3) * 2;
+        int it = pair, cc = 0;                                            // item and chunk being stored
+        int k = it < items ? item_k0(it) : 0, k1 = it < items ? item_k1(it) : 0;
+        bool alive = true, fresh = true;                                  // fresh: first chunk of an item
+        while (it < items && alive) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                if (it >= items) break;
+                const int s = cc % WW_STAGES;
+                if (FMT == WW_W4A && (fresh || k % p.G == 0)) {
+                    const int n = item_n(it) + 16 * ch;
+                    const uint16_t* zp = p.zeros + static_cast<int64_t>(k / p.G) * p.N + n;
+                    uint4 z[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) z[i] = n < p.N ? __ldg(reinterpret_cast<const uint4*>(zp) + i) : make_uint4(0, 0, 0, 0);
+                    const uint32_t zz[8] = {z[0].x, z[0].y, z[0].z, z[0].w, z[1].x, z[1].y, z[1].z, z[1].w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) bias[i] = ww_hfma2(zz[i], 0x3c003c00u, 0x64006400u);   // 1024 + z
+                }
+                if (!ptx::mbar_wait(empty(s), ((cc / WW_STAGES) & 1) ^ 1, abort_flag, p.status)) { alive = false; break; }
+                uint8_t* at = smem + s * WW_STAGE_BYTES + flip * (WW_A_BYTES / 2);
+                auto put = [&](int kk, uint4 a, uint4 b) {
+                    uint8_t* base = at + kk * 128;
+                    *reinterpret_cast<uint4*>(base + (((c2 + flip) ^ (kk & 7)) << 4)) = flip ? b : a;
+                    *reinterpret_cast<uint4*>(base + (((c2 + 1 - flip) ^ (kk & 7)) << 4)) = flip ? a : b;
+                };
+#pragma unroll
+                for (int i = 0; i < LOADS; ++i) {
+                    const uint4 v = w[x][i];
+                    const int row = kr + 16 * i;
+                    if (FMT == WW_W8) {
+                        uint4 a, b;
+                        ptx::i8x4_to_f16(v.x, a.x, a.y); ptx::i8x4_to_f16(v.y, a.z, a.w);
+                        ptx::i8x4_to_f16(v.z, b.x, b.y); ptx::i8x4_to_f16(v.w, b.z, b.w);
+                        put(row, a, b);
+                    } else {
+                        uint32_t e[4][2], o[4][2];
+                        ww_nibbles<FMT == WW_W4A>(v.x, bias[0], bias[1], e[0], o[0]);
+                        ww_nibbles<FMT == WW_W4A>(v.y, bias[2], bias[3], e[1], o[1]);
+                        ww_nibbles<FMT == WW_W4A>(v.z, bias[4], bias[5], e[2], o[2]);
+                        ww_nibbles<FMT == WW_W4A>(v.w, bias[6], bias[7], e[3], o[3]);
+                        put(2 * row, make_uint4(e[0][0], e[0][1], e[1][0], e[1][1]), make_uint4(e[2][0], e[2][1], e[3][0], e[3][1]));
+                        put(2 * row + 1, make_uint4(o[0][0], o[0][1], o[1][0], o[1][1]), make_uint4(o[2][0], o[2][1], o[3][0], o[3][1]));
+                    }
+                }
+                load(w[x]);
+                ptx::fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(a_full(s), 0));
+                ++cc;
+                k += WW_CHUNK;
+                fresh = k >= k1;
+                if (fresh) {
+                    it += n_pairs;
+                    if (it < items) { k = item_k0(it); k1 = item_k1(it); }
+                }
+            }
+        }
+    } else {
+        ptx::fewer_registers<WW_REG_REST>();
+        if (warp == 12 && ptx::elect_one()) {
+            // ---- activation tiles: this CTA's half of the rows, high and low ----
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            const uint32_t bytes = static_cast<uint32_t>(p.rows / 2) * WW_CHUNK * 2;
+            int cc = 0;
+            bool ok = true;
+            for (int it = pair; it < items && ok; it += n_pairs) {
+                const int k1 = item_k1(it), m = item_m(it) + static_cast<int>(rank) * (p.rows / 2);
+                for (int k = item_k0(it); k < k1; k += WW_CHUNK, ++cc) {
+                    const int s = cc % WW_STAGES;
+                    if (!ptx::mbar_wait(empty(s), ((cc / WW_STAGES) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
+                    const uint32_t leader = ptx::mapa_shared(b_full(s), 0);
+                    if (rank == 0) ptx::mbar_expect_tx(b_full(s), 4 * bytes);           // both CTAs' bytes
+                    const uint32_t dst = ptx::smem_u32(smem + s * WW_STAGE_BYTES + WW_A_BYTES);
+                    ptx::tma_load_2d_pair(dst, &tmHi, k, m, leader);
+                    ptx::tma_load_2d_pair(dst + WW_B_BYTES, &tmLo, k, m, leader);
+                }
+            }
+            // the last stages' commits have arrived in this CTA before it leaves
+            for (int j = 0; j < WW_STAGES && ok; ++j) {
+                const int c = cc - 1 - j;
+                if (c >= 0) ok = ptx::mbar_wait(empty(c % WW_STAGES), (c / WW_STAGES) & 1, abort_flag, p.status);
+            }
+        } else if (warp == 13 && rank == 0 && ptx::elect_one()) {
+            // ---- MMA issuer ----
+            const uint32_t idesc = ww_idesc(p.rows);
+            int cc = 0;
+            uint32_t units = 0;
+            bool ok = true;
+            for (int it = pair; it < items && ok; it += n_pairs) {
+                const int k1 = item_k1(it);
+                for (int k = item_k0(it); k < k1; k += WW_CHUNK, ++cc) {
+                    const int s = cc % WW_STAGES;
+                    ok = ptx::mbar_wait(b_full(s), (cc / WW_STAGES) & 1, abort_flag, p.status) &&
+                         ptx::mbar_wait(a_full(s), (cc / WW_STAGES) & 1, abort_flag, p.status);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint32_t sa = ptx::smem_u32(smem + s * WW_STAGE_BYTES), sb = sa + WW_A_BYTES;
+                    // accumulators begin and end at multiples of p.unit (32, 64 or 128): two half-chunks of 32 k
+#pragma unroll
+                    for (int hc = 0; hc < 2; ++hc) {
+                        const int kk = k + 32 * hc;
+                        const bool first = kk % p.unit == 0, last = (kk + 32) % p.unit == 0 || kk + 32 >= k1;
+                        const int b = units & 1;
+                        if (first) {
+                            ok = ptx::mbar_wait(t_empty(b), ((units >> 1) & 1) ^ 1, abort_flag, p.status);
+                            if (!ok) break;
+                            ptx::tc_fence_after();
+                        }
+#pragma unroll
+                        for (int pass = 0; pass < 2; ++pass)              // the low halves first
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                const int step = 2 * hc + j;
+                                ptx::mma_f16_ss_pair(tmem + 256 * b, ptx::smem_desc_sw128(sa + step * 2048, WW_A_BYTES / 2, 1024),
+                                                     ptx::smem_desc_sw128(sb + (1 - pass) * WW_B_BYTES + step * 32, 16, 1024), idesc,
+                                                     (first && pass == 0 && j == 0) ? 0u : 1u);
+                            }
+                        if (last) {
+                            ptx::tc_commit_pair(ptx::mapa_shared(t_full(b), 0));
+                            ptx::tc_commit_pair(ptx::mapa_shared(t_full(b), 1));
+                            ++units;
+                        }
+                    }
+                    if (!ok) break;
+                    ptx::tc_commit_pair(ptx::mapa_shared(empty(s), 0));   // the stage is free in both CTAs
+                    ptx::tc_commit_pair(ptx::mapa_shared(empty(s), 1));
+                }
+            }
+        }
+    }
+
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::cluster_sync_all();                                 // neither CTA frees memory the pair may still touch
+    if (warp == 14) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc_pair(tmem, 512);
+    }
+}
+
+// the parts of a split K, added in order
+__global__ void __launch_bounds__(256)
+wide_reduce_kernel(const float* __restrict__ part, float* __restrict__ C, int64_t total, int splits, float alpha, float beta) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int64_t i = (blockIdx.x * static_cast<int64_t>(256) + threadIdx.x) * 4;
+    if (i >= total) return;
+    float4 v = *reinterpret_cast<const float4*>(part + i);
+    for (int s = 1; s < splits; ++s) {
+        const float4 x = *reinterpret_cast<const float4*>(part + s * total + i);
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+    }
+    v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha;
+    if (beta != 0.0f) {
+        const float4 o = *reinterpret_cast<const float4*>(C + i);
+        v.x = fmaf(beta, o.x, v.x); v.y = fmaf(beta, o.y, v.y); v.z = fmaf(beta, o.z, v.z); v.w = fmaf(beta, o.w, v.w);
+    }
+    *reinterpret_cast<float4*>(C + i) = v;
+}
+
+// ---- host side ----------------------------------------------------------------------------
+
+struct WidePlan { int rows, m_blocks, splits; };
+
+// Rows per tile and K splits: the pass over the longest pair's work.  A tile of r rows costs r tensor cycles per 16 k and
+// pass (never less than about 64: the converters' pace), a split its partial sums (and the launch that adds them).
+static WidePlan wide_plan(int M, int N, int K, int pairs, size_t part_floats) {
+    WidePlan best{32, ceil_div(M, 32), 1};
+    double best_cost = -1;
+    const int col_tiles = ceil_div(N, WW_COLS), k_blocks = ceil_div(K, 128);
+    for (int rows = 32; rows <= WW_MAX_ROWS; rows += 32) {
+        const int mb = ceil_div(M, rows);
+        if (rows > 32 && mb == ceil_div(M, rows - 32)) continue;            // fewer rows a tile do as well
+        for (int s = 1; s <= 16 && s <= k_blocks; ++s) {
+            if (s > 1 && static_cast<size_t>(s) * M * N > part_floats) break;
+            const int64_t waves = (static_cast<int64_t>(mb) * col_tiles * s + pairs - 1) / pairs;
+            const double cost = static_cast<double>(waves) * (ceil_div(k_blocks, s) * 16.0 * std::max(rows + 8, 72) + 6.0 * rows + 1500) +
+                                (s > 1 ? 6000.0 + 0.0012 * s * M * N : 0.0);
+            if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = WidePlan{rows, mb, s}; }
+        }
+    }
+    return best;
+}
+
+// fmt: 0 symmetric int4, 1 asymmetric int4, 2 int8 per channel
+bool wo_wide_ok(int fmt, int M, int N, int K, int G) {
+    if (M < 1 || N < 16 || (N % 16) != 0 || K < 64 || (K % 64) != 0) return false;
+    if (fmt == WW_W8) return true;
+    if (fmt == WW_W4A && (G % 64) != 0) return false;                       // one zero-point per column and chunk
+    if (K % G) return false;
+    return G == 32 || G == 64 || (G >= 128 && (G % 128) == 0);
+}
+
+bool wo_wide_prefer(int fmt, int M, int N, int K, int G) {
+    if (!wo_wide_ok(fmt, M, N, K, G)) return false;
+    if (knobs().wo_wide_min_m > 0) return M >= knobs().wo_wide_min_m;
+    return M > 32;
+}
+
+template <int FMT>
+static int launch_wide(lhb_ctx* ctx, const TensorMap& hi, const TensorMap& lo, const WideParams& p, cudaStream_t st) {
+    auto kern = gemm_wo_wide_kernel<FMT>;
+    static bool attr_set[64] = {};
+    if (!attr_set[ctx->device & 63]) {
+        LHB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(WW_SMEM)));
+        attr_set[ctx->device & 63] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    const int items = p.m_blocks * p.col_tiles * p.splits;
+    cfg.gridDim = dim3(2 * std::max(1, std::min(ctx->sm_count / 2, items)), 1, 1);
+    cfg.blockDim = dim3(WW_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = WW_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = knobs().pdl ? 2 : 1;
+    LHB_CUDA(cudaLaunchKernelEx(&cfg, kern, hi, lo, p));
+    return LHB_OK;
+}
+
+// scratch: [high halves][low halves][row factors][partial sums], for as many rows at a time as leave half of it for the sums
+int launch_wo_wide(lhb_ctx* ctx, int fmt, const float* A, const void* B, const void* scales, const void* zeros, float* C, int M,
+                   int N, int K, int G, float alpha, float beta, cudaStream_t st, int prologue, const float* gamma, float eps) {
+    if (!wo_wide_ok(fmt, M, N, K, G)) return LHB_ERR_UNSUPPORTED;
+    const size_t row_bytes = static_cast<size_t>(K) * 4 + 4;
+    const size_t digit_budget = ctx->scratch_bytes / 2;
+    const int64_t fit = static_cast<int64_t>((digit_budget - std::min<size_t>(digit_budget, 4096)) / row_bytes) / 256 * 256;
+    if (fit < 256) return LHB_ERR_UNSUPPORTED;
+    const int64_t row_len = (prologue == 2) ? 2 * static_cast<int64_t>(K) : K;
+    for (int m0 = 0; m0 < M; m0 += static_cast<int>(std::min<int64_t>(fit, M))) {
+        const int m = static_cast<int>(std::min<int64_t>(fit, M - m0));
+        uint8_t* base = static_cast<uint8_t*>(ctx->scratch);
+        __half* hi = reinterpret_cast<__half*>(base);
+        __half* lo = hi + static_cast<size_t>(m) * K;
+        float* inv = reinterpret_cast<float*>(lo + static_cast<size_t>(m) * K);
+        const size_t used = (static_cast<size_t>(m) * row_bytes + 1023) / 1024 * 1024;
+        float* part = reinterpret_cast<float*>(base + used);
+        cudaLaunchConfig_t dc = {};
+        cudaLaunchAttribute pdl[1];
+        pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        pdl[0].val.programmaticStreamSerializationAllowed = 1;
+        dc.gridDim = dim3(m, 1, 1);
+        dc.blockDim = dim3(512, 1, 1);
+        dc.stream = st;
+        dc.attrs = pdl;
+        dc.numAttrs = knobs().pdl ? 1 : 0;
+        LHB_CUDA(cudaLaunchKernelEx(&dc, wide_digits_kernel, A + m0 * row_len, K, hi, lo, inv, prologue, gamma, eps));
+        const WidePlan pl = wide_plan(m, N, K, std::max(1, ctx->sm_count / 2), (ctx->scratch_bytes - used) / sizeof(float));
+        TensorMap tmHi, tmLo;
+        if (int e = get_tensor_map_2d_f16_sw128(ctx, hi, m, K, static_cast<uint64_t>(K) * 2, pl.rows / 2, WW_CHUNK, &tmHi)) return e;
+        if (int e = get_tensor_map_2d_f16_sw128(ctx, lo, m, K, static_cast<uint64_t>(K) * 2, pl.rows / 2, WW_CHUNK, &tmLo)) return e;
+        WideParams p{};
+        p.B = static_cast<const uint8_t*>(B); p.scales = scales; p.zeros = static_cast<const uint16_t*>(zeros);
+        p.C = C + static_cast<int64_t>(m0) * N; p.part = part; p.inv_scale = inv;
+        p.M = m; p.N = N; p.K = K; p.G = fmt == WW_W8 ? K : G;
+        p.unit = fmt == WW_W8 ? 128 : std::min(G, 128);
+        p.rows = pl.rows; p.m_blocks = pl.m_blocks; p.col_tiles = ceil_div(N, WW_COLS); p.splits = pl.splits;
+        p.alpha = alpha; p.beta = beta; p.status = ctx->status_word;
+        const int e = fmt == WW_W4 ? launch_wide<WW_W4>(ctx, tmHi, tmLo, p, st)
+                      : fmt == WW_W4A ? launch_wide<WW_W4A>(ctx, tmHi, tmLo, p, st) : launch_wide<WW_W8>(ctx, tmHi, tmLo, p, st);
+        if (e) return e;
+        if (pl.splits > 1) {
+            const int64_t total = static_cast<int64_t>(m) * N;
+            dc.gridDim = dim3(static_cast<unsigned>(ceil_div64(total, 1024)), 1, 1);
+            dc.blockDim = dim3(256, 1, 1);
+            LHB_CUDA(cudaLaunchKernelEx(&dc, wide_reduce_kernel, static_cast<const float*>(part), p.C, total, pl.splits, alpha, beta));
+        }
+    }
+    return LHB_OK;
+}
+
+}  // namespace lhb

@@ -20,7 +20,7 @@
 //                that a key's two scales are read once for two rows by an 8-byte load with four addresses a warp (the
 //                row-per-thread layout reads them with broadcasts, one wavefront per key, scale and warp:
 //                shared memory then is the bound), and adds the previous tile's O to its registers;
-//   warps 8-11   int8 -> fp16: 128-bit loads of whole pages straight to registers, one operand ahead, an
+//   warps 8-11   int8 -> fp16: 128-bit loads of whole pages straight to registers, one tile ahead, an
 //                exclusive-or, a byte permute and a subtraction per two values, 128-byte-swizzled stores.  K and V
 //                lie in shared memory as [token][d] alike, K read K-major, V MN-major;
 //   warp 12      MMA issuer: PV(j), then QK(j + 2) into the S it has freed.
@@ -83,44 +83,6 @@ __device__ __forceinline__ float pf_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// two fp32 -> packed fp16, `lo` in the low half
-__device__ __forceinline__ uint32_t pf_pack(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-// four int8 -> two packed fp16 pairs: a byte b ^ 0x80 under the exponent byte 0x64 is 1024 + 128 + b
-__device__ __forceinline__ void pf_cvt4(uint32_t w, uint32_t& a, uint32_t& b) {
-    const uint32_t u = w ^ 0x80808080u;
-    a = __byte_perm(u, 0x64646464u, 0x4140);
-    b = __byte_perm(u, 0x64646464u, 0x4342);
-    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(a) : "r"(0x64806480u));
-    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(b) : "r"(0x64806480u));
-}
-// the part of |x| that fits fp16's 11 bits, by truncation; the rest is exact in fp32
-__device__ __forceinline__ float pf_high(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
-
-// two fp32 operations in one instruction
-__device__ __forceinline__ float2 pf_mul2(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
-    return d;
-}
-__device__ __forceinline__ float2 pf_add2(float2 a, float2 b) {
-    float2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
-    return d;
-}
-__device__ __forceinline__ float2 pf_fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t&>(d))
-        : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
-    return d;
-}
-template <int N> __device__ __forceinline__ void pf_more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void pf_fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-
 // keys [lo, hi] that the query at position `pos` sees (empty when lo > hi); lo and hi do not fall as pos rises
 __device__ __forceinline__ void pf_visible(const PrefillParams& p, int pos, int len, int& lo, int& hi) {
     lo = 0;
@@ -225,12 +187,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
             float4 v = q_row(r);
             if (row_bad[r]) v = make_float4(0.f, 0.f, 0.f, 0.f);                  // the row's output becomes NaN at the end
             v.x *= scl; v.y *= scl; v.z *= scl; v.w *= scl;
-            const float hx = pf_high(v.x), hy = pf_high(v.y), hz = pf_high(v.z), hw = pf_high(v.w);
+            const float hx = ptx::f16_high(v.x), hy = ptx::f16_high(v.y), hz = ptx::f16_high(v.z), hw = ptx::f16_high(v.w);
             // elements 4 * lane .. +3: half lane / 16, 16-byte chunk (lane % 16) / 2, 8 bytes into it
             const int off = (lane >> 4) * PF_HALF_BYTES + r * 128 + (((((lane & 15) >> 1) ^ (r & 7))) << 4) + (lane & 1) * 8;
-            *reinterpret_cast<uint2*>(q_sm + off) = make_uint2(pf_pack(hx, hy), pf_pack(hz, hw));
+            *reinterpret_cast<uint2*>(q_sm + off) = make_uint2(ptx::pack_f16(hx, hy), ptx::pack_f16(hz, hw));
             *reinterpret_cast<uint2*>(q_sm + PF_TILE_BYTES + off) =
-                make_uint2(pf_pack(v.x - hx, v.y - hy), pf_pack(v.z - hz, v.w - hw));
+                make_uint2(ptx::pack_f16(v.x - hx, v.y - hy), ptx::pack_f16(v.z - hz, v.w - hw));
         }
         ptx::fence_proxy_async_smem();
     }
@@ -240,7 +202,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
     const uint32_t tmem = *tmem_slot;                            // columns: S / P buffers at 0 and 128, O buffers at 256 and 384
 
     if (warp < 8) {
-        pf_more_registers<PF_REG_SOFTMAX>();
+        ptx::more_registers<PF_REG_SOFTMAX>();
         // ---- softmax: rows ra and ra + 8, columns 8 i + 2 (lane % 4) and + 1 ----
         const int row16 = 32 * (warp & 3) + 16 * (warp >> 2);    // first of the warp's rows = TMEM lanes
         const int ra = row16 + (lane >> 2), rb = ra + 8, col = 2 * (lane & 3);
@@ -275,8 +237,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int k = c0 / 4 + 2 * i;
-                    o[k] = pf_fma2(o[k], aa, make_float2(__uint_as_float(t[4 * i]), __uint_as_float(t[4 * i + 1])));
-                    o[k + 1] = pf_fma2(o[k + 1], ab, make_float2(__uint_as_float(t[4 * i + 2]), __uint_as_float(t[4 * i + 3])));
+                    o[k] = ptx::fma2(o[k], aa, make_float2(__uint_as_float(t[4 * i]), __uint_as_float(t[4 * i + 1])));
+                    o[k + 1] = ptx::fma2(o[k + 1], ab, make_float2(__uint_as_float(t[4 * i + 2]), __uint_as_float(t[4 * i + 3])));
                 }
             }
             return true;
@@ -290,23 +252,25 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
             const float* pr = par + (j & 3) * PF_PARAM_FLOATS + col;
             const int key0 = (page_base + j * 8) * PF_BS;
             const uint32_t s_addr = base + 128 * b;
+            const uint4 vmax = *reinterpret_cast<const uint4*>(pr - col + 2 * PF_KEYS), valid = *reinterpret_cast<const uint4*>(pr - col + 2 * PF_KEYS + 4);
+            const bool masked = key0 < all_lo || key0 + PF_KEYS - 1 > all_hi || (valid.x & valid.y & valid.z & valid.w) != 0xffffffffu;
             uint32_t y[64];                                      // per 8 columns: row a col, col + 1, row b col, col + 1
             ptx::tmem_ld_16x32(s_addr, y);
-            ptx::tmem_ld_16x32(s_addr + 32, y + 16);
-            ptx::tmem_ld_16x32(s_addr + 64, y + 32);
-            ptx::tmem_ld_16x32(s_addr + 96, y + 48);
-            const uint4 vmax = *reinterpret_cast<const uint4*>(pr - col + 2 * PF_KEYS), valid = *reinterpret_cast<const uint4*>(pr - col + 2 * PF_KEYS + 4);
-            ptx::tmem_ld_wait();
-            // scores in base 2
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float2 ks = *reinterpret_cast<const float2*>(pr + 8 * i);
-                const float2 a = pf_mul2(make_float2(__uint_as_float(y[4 * i]), __uint_as_float(y[4 * i + 1])), ks);
-                const float2 c = pf_mul2(make_float2(__uint_as_float(y[4 * i + 2]), __uint_as_float(y[4 * i + 3])), ks);
-                y[4 * i] = __float_as_uint(a.x); y[4 * i + 1] = __float_as_uint(a.y);
-                y[4 * i + 2] = __float_as_uint(c.x); y[4 * i + 3] = __float_as_uint(c.y);
+            for (int c0 = 0; c0 < PF_KEYS; c0 += 32) {
+                ptx::tmem_ld_wait();                             // also keeps the scales of later columns from being loaded early
+                if (c0 + 32 < PF_KEYS) ptx::tmem_ld_16x32(s_addr + c0 + 32, y + c0 / 2 + 16);
+                // scores in base 2
+#pragma unroll
+                for (int i = c0 / 8; i < c0 / 8 + 4; ++i) {
+                    const float2 ks = *reinterpret_cast<const float2*>(pr + 8 * i);
+                    const float2 a = ptx::mul2(make_float2(__uint_as_float(y[4 * i]), __uint_as_float(y[4 * i + 1])), ks);
+                    const float2 c = ptx::mul2(make_float2(__uint_as_float(y[4 * i + 2]), __uint_as_float(y[4 * i + 3])), ks);
+                    y[4 * i] = __float_as_uint(a.x); y[4 * i + 1] = __float_as_uint(a.y);
+                    y[4 * i + 2] = __float_as_uint(c.x); y[4 * i + 3] = __float_as_uint(c.y);
+                }
             }
-            if (key0 < all_lo || key0 + PF_KEYS - 1 > all_hi || (valid.x & valid.y & valid.z & valid.w) != 0xffffffffu) {
+            if (masked) {
                 const uint32_t bits[4] = {valid.x, valid.y, valid.z, valid.w};
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
@@ -337,25 +301,26 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
             float2 la = make_float2(0.f, 0.f), lb = la;
 #pragma unroll
             for (int s = 0; s < 8; ++s) {                        // 16 keys: an MMA step of P
+                const uint32_t* yc = y + 8 * s;
                 uint32_t w[8];                                   // columns 0-7 high halves, 8-15 low halves; rows a, b of each four
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const int i = 2 * s + u;
-                    const float2 vs = *reinterpret_cast<const float2*>(pr + PF_KEYS + 8 * i);
-                    float2 a = pf_add2(make_float2(__uint_as_float(y[4 * i]), __uint_as_float(y[4 * i + 1])), ea2);
-                    float2 c = pf_add2(make_float2(__uint_as_float(y[4 * i + 2]), __uint_as_float(y[4 * i + 3])), eb2);
+                    const int i = u;
+                    const float2 vs = *reinterpret_cast<const float2*>(pr + PF_KEYS + 16 * s + 8 * u);
+                    float2 a = ptx::add2(make_float2(__uint_as_float(yc[4 * i]), __uint_as_float(yc[4 * i + 1])), ea2);
+                    float2 c = ptx::add2(make_float2(__uint_as_float(yc[4 * i + 2]), __uint_as_float(yc[4 * i + 3])), eb2);
                     a.x = pf_exp2(a.x); a.y = pf_exp2(a.y); c.x = pf_exp2(c.x); c.y = pf_exp2(c.y);
-                    la = pf_add2(la, a);
-                    lb = pf_add2(lb, c);
-                    a = pf_mul2(a, vs);
-                    c = pf_mul2(c, vs);
-                    const float2 ha = make_float2(pf_high(a.x), pf_high(a.y)), hc = make_float2(pf_high(c.x), pf_high(c.y));
-                    a = pf_fma2(ha, minus1, a);
-                    c = pf_fma2(hc, minus1, c);
-                    w[2 * u] = pf_pack(ha.x, ha.y);
-                    w[2 * u + 1] = pf_pack(hc.x, hc.y);
-                    w[4 + 2 * u] = pf_pack(a.x, a.y);
-                    w[4 + 2 * u + 1] = pf_pack(c.x, c.y);
+                    la = ptx::add2(la, a);
+                    lb = ptx::add2(lb, c);
+                    a = ptx::mul2(a, vs);
+                    c = ptx::mul2(c, vs);
+                    const float2 ha = make_float2(ptx::f16_high(a.x), ptx::f16_high(a.y)), hc = make_float2(ptx::f16_high(c.x), ptx::f16_high(c.y));
+                    a = ptx::fma2(ha, minus1, a);
+                    c = ptx::fma2(hc, minus1, c);
+                    w[2 * u] = ptx::pack_f16(ha.x, ha.y);
+                    w[2 * u + 1] = ptx::pack_f16(hc.x, hc.y);
+                    w[4 + 2 * u] = ptx::pack_f16(a.x, a.y);
+                    w[4 + 2 * u + 1] = ptx::pack_f16(c.x, c.y);
                 }
                 ptx::tmem_st_16x16(s_addr + 16 * s, w);
             }
@@ -394,33 +359,40 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
             }
         }
     } else if (warp < 12) {
-        pf_fewer_registers<PF_REG_CONVERT>();
+        ptx::fewer_registers<PF_REG_CONVERT>();
         // ---- converters: warp cw owns pages 2 cw and 2 cw + 1 of every tile, thread ct the scales of token ct ----
-        const int cw = warp - 8, ct = threadIdx.x - 256;
+        const int cw = warp - 8, ct = 32 * cw + lane;
         const int last_page = min((len + PF_BS - 1) / PF_BS, p.max_blocks) - 1;
-        auto page_row = [&](int page) {                          // first row of a page of this head; -1: masked
-            if (page > last_page) return int64_t(-1);
-            const int blk = table[page];
-            return (blk >= 0 && blk < p.num_blocks) ? (static_cast<int64_t>(blk) * p.n_kv_heads + kvh) * PF_BS : int64_t(-1);
+        // ids of this warp's two pages of a tile, fetched a tile before their rows are loaded; -1: masked
+        int2 ids = make_int2(-1, -1);
+        auto fetch_ids = [&](int j) {
+            const int pg = page_base + j * 8 + 2 * cw;
+            ids.x = pg <= last_page ? __ldg(table + pg) : -1;
+            ids.y = pg + 1 <= last_page ? __ldg(table + pg + 1) : -1;
         };
-        int64_t row_a = -1, row_b = -1;                          // the two pages, of the tile being loaded
-        auto load = [&](uint4 (&w)[8], const int8_t* pool) {     // 4 tokens per instruction, 512 contiguous bytes
+        int blk_a = -1, blk_b = -1;                              // the two pages of the tile being loaded
+        auto page_row = [&](int blk) { return (static_cast<int64_t>(blk) * p.n_kv_heads + kvh) * PF_BS; };   // first row of a page of this head
+        uint4 w[8];                                              // the operand that is stored next: K(j), V(j), K(j + 1), ...
+        auto load = [&](const int8_t* pool) {                                      // 4 tokens per instruction, 512 contiguous bytes
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int64_t row = i < 4 ? row_a : row_b;
-                w[i] = row >= 0 ? __ldg(reinterpret_cast<const uint4*>(pool + row * PF_D + (i & 3) * 512 + lane * 16)) : make_uint4(0, 0, 0, 0);
+            for (int x = 0; x < 2; ++x) {
+                const int blk = x ? blk_b : blk_a;
+                const int8_t* src = pool + page_row(blk) * PF_D + lane * 16;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    w[4 * x + i] = blk >= 0 ? __ldg(reinterpret_cast<const uint4*>(src + i * 512)) : make_uint4(0, 0, 0, 0);
             }
         };
         // 16 values of token tok, d = 16 ch .. +15: half ch / 4, chunks 2 (ch % 4) and + 1, swizzled with the token;
         // lanes of the two halves store their chunks in opposite order (no bank is met twice)
         const int ch = lane & 7, flip = ch >> 2;
-        auto store = [&](const uint4 (&w)[8], uint8_t* tile) {
+        auto store = [&](uint8_t* tile) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int tok = cw * 32 + i * 4 + (lane >> 3);
                 uint4 a, b;
-                pf_cvt4(w[i].x, a.x, a.y); pf_cvt4(w[i].y, a.z, a.w);
-                pf_cvt4(w[i].z, b.x, b.y); pf_cvt4(w[i].w, b.z, b.w);
+                ptx::i8x4_to_f16(w[i].x, a.x, a.y); ptx::i8x4_to_f16(w[i].y, a.z, a.w);
+                ptx::i8x4_to_f16(w[i].z, b.x, b.y); ptx::i8x4_to_f16(w[i].w, b.z, b.w);
                 uint8_t* base = tile + flip * PF_HALF_BYTES + tok * 128;
                 const int c2 = (ch & 3) * 2;
                 *reinterpret_cast<uint4*>(base + (((c2 + flip) ^ (tok & 7)) << 4)) = flip ? b : a;
@@ -428,24 +400,23 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
             }
         };
         const float s_scale = __uint_as_float(static_cast<uint32_t>(254 - q_exp) << 23) * p.scale_log2e;
-        uint4 w[8];                                              // the operand that is stored next: K(j), V(j), K(j + 1), ...
         float ks = 0.0f, vs = 0.0f;
         bool ok = false;
-        auto load_k = [&](int j) {
-            const int pg = page_base + j * 8 + 2 * cw;
-            row_a = page_row(pg);
-            row_b = page_row(pg + 1);
-            load(w, p.Kp);
-            const int64_t row = (lane & 16) ? row_b : row_a;     // token ct = 32 cw + lane
-            ok = row >= 0 && (page_base + j * 8) * PF_BS + ct < len;
-            if (ok) { ks = __ldg(p.Ks + row + (ct & 15)); vs = __ldg(p.Vs + row + (ct & 15)); }
+        auto load_k = [&](int j) {                               // K and the scales of tile j, then the ids of the next
+            blk_a = ids.x < p.num_blocks ? ids.x : -1;           // negative ids stay what they are
+            blk_b = ids.y < p.num_blocks ? ids.y : -1;
+            load(p.Kp);
+            const int blk = (lane & 16) ? blk_b : blk_a;         // token ct = 32 cw + lane
+            ok = blk >= 0 && (page_base + j * 8) * PF_BS + ct < len;
+            if (ok) { ks = __ldg(p.Ks + page_row(blk) + (ct & 15)); vs = __ldg(p.Vs + page_row(blk) + (ct & 15)); }
+            fetch_ids(j + 1);
         };
-        if (n_tiles > 0) load_k(0);
+        if (n_tiles > 0) { fetch_ids(0); load_k(0); }
         for (int j = 0; j < n_tiles; ++j) {
             const int b = j & 1, parity = ((j >> 1) & 1) ^ 1;
             if (!ptx::mbar_wait(k_empty(b), parity, abort_flag, p.status)) break;
-            store(w, k_sm + b * PF_TILE_BYTES);
-            load(w, p.Vp);
+            store(k_sm + b * PF_TILE_BYTES);
+            load(p.Vp);                                          // in flight while the fence drains the stores
             float* pr = par + (j & 3) * PF_PARAM_FLOATS;
             const unsigned vbits = __reduce_max_sync(0xffffffffu, ok ? __float_as_uint(vs) & 0x7fffffffu : 0u);
             const unsigned valid = __ballot_sync(0xffffffffu, ok);
@@ -456,17 +427,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
                 reinterpret_cast<unsigned*>(pr)[2 * PF_KEYS + 4 + cw] = valid;
             }
             __syncwarp();
-            ptx::fence_proxy_async_smem();
             ptx::mbar_arrive(par_full(j & 3));
+            ptx::fence_proxy_async_smem();
             ptx::mbar_arrive(k_full(b));
             if (!ptx::mbar_wait(v_empty(b), parity, abort_flag, p.status)) break;
-            store(w, v_sm + b * PF_TILE_BYTES);
+            store(v_sm + b * PF_TILE_BYTES);
             if (j + 1 < n_tiles) load_k(j + 1);
             ptx::fence_proxy_async_smem();
             ptx::mbar_arrive(v_full(b));
         }
     } else {
-        pf_fewer_registers<PF_REG_ISSUE>();
+        ptx::fewer_registers<PF_REG_ISSUE>();
         if (warp == 12 && ptx::elect_one()) {
             // ---- MMA issuer ----
             const uint32_t qa = ptx::smem_u32(q_sm), ka = ptx::smem_u32(k_sm), va = ptx::smem_u32(v_sm);

@@ -230,6 +230,15 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
+// 32 lanes x 16 columns of 32-bit
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
 // 16 lanes x 32 columns of 32-bit in the layout of an MMA accumulator fragment: per 8 columns, thread i gets lane
 // i / 4, columns 2 (i % 4) and + 1, then the same columns of lane i / 4 + 8
 __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
@@ -239,6 +248,11 @@ __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
 }
 // 16 lanes x 16 columns: per 4 columns, thread i writes column i % 4 of lane i / 4, then of lane i / 4 + 8
 __device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t (&r)[8]) {
@@ -323,10 +337,62 @@ __device__ __forceinline__ void mma_f8_ss_pair(uint32_t tmem_d, uint64_t desc_a,
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+__device__ __forceinline__ void mma_f16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // arrives on a barrier (shared::cluster address, own or peer CTA) when the pair's MMAs issued so far are done
 __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
                  : "memory");
+}
+
+// ---- register budget of a warpgroup (all of its four warps; the launch's total is never exceeded) --------------
+template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// ---- packed arithmetic -------------------------------------------------------------------------
+
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+    return d;
+}
+// two fp32 -> packed fp16, `lo` in the low half
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// the part of |x| that fits fp16's 11 bits, by truncation; the rest is exact in fp32
+__device__ __forceinline__ float f16_high(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
+// four int8 -> two packed fp16 pairs, exactly: a byte b ^ 0x80 under the exponent byte 0x64 is 1024 + 128 + b
+__device__ __forceinline__ void i8x4_to_f16(uint32_t w, uint32_t& a, uint32_t& b) {
+    const uint32_t u = w ^ 0x80808080u;
+    a = __byte_perm(u, 0x64646464u, 0x4140);
+    b = __byte_perm(u, 0x64646464u, 0x4342);
+    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(a) : "r"(0x64806480u));
+    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(b) : "r"(0x64806480u));
 }
 
 }  // namespace ptx

@@ -178,7 +178,12 @@ int lhb_gemm_w4a16_asym(lhb_ctx* ctx, const float* A, const uint8_t* Bp, const u
     if (M == 0) return LHB_OK;
     cudaStream_t st = as_stream(stream);
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (w4a16_asym_fast_ok(M, N, K, group_size) && al16(A) && al16(Bp) && al16(scales_h) && al16(zeros_h) && al16(C))
+    const bool al = al16(A) && al16(Bp) && al16(scales_h) && al16(zeros_h) && al16(C);
+    if (al && wo_wide_prefer(1, M, N, K, group_size)) {
+        const int e = launch_wo_wide(ctx, 1, A, Bp, scales_h, zeros_h, C, M, N, K, group_size, alpha, beta, st);
+        if (e != LHB_ERR_UNSUPPORTED) return e;
+    }
+    if (w4a16_asym_fast_ok(M, N, K, group_size) && al)
         return launch_w4a16_asym_fast(ctx, A, Bp, scales_h, zeros_h, C, M, N, K, group_size, alpha, beta, st);
     return launch_w4a16_asym_generic(A, Bp, scales_h, zeros_h, C, M, N, K, group_size, alpha, beta, st);
 }

@@ -96,6 +96,13 @@ int get_tensor_map_2d_f16(lhb_ctx* ctx, const void* base, uint64_t rows, uint64_
                              box_cols, false, out);
 }
 
+// fp16 with the 128-byte swizzle (box_cols * 2 == 128)
+int get_tensor_map_2d_f16_sw128(lhb_ctx* ctx, const void* base, uint64_t rows, uint64_t cols,
+                                uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols, TensorMap* out) {
+    return get_tensor_map_2d(ctx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, base, rows, cols, pitch_bytes, box_rows,
+                             box_cols, true, out);
+}
+
 }  // namespace lhb
 
 namespace lhb {
@@ -108,6 +115,7 @@ const Knobs& knobs() {
         };
         v.pdl = num("LHB_PDL", 1) != 0;
         v.w4tc_min_m = std::max(1, num("LHB_W4TC_MIN_M", 9));
+        v.wo_wide_min_m = std::max(0, num("LHB_WO_WIDE_MIN_M", 0));
         v.w4tc_stream_k = num("LHB_W4TC_SPLIT", 0) == 1;
         v.w4tc_ctas = std::max(0, num("LHB_W4TC_CTAS", 0));
         v.w4tc_coop = num("LHB_W4TC_COOP", 1) != 0;

@@ -1,0 +1,101 @@
+"""GPU parity of the weight-only GEMMs with many rows (int4 groups, asymmetric int4, int8 per channel) at the edges
+of their tiles: ragged row and column tiles, groups below, at and above an accumulator's 128 k, a last half
+block of K, K split over CTA pairs, several tiles per pair.  Outputs must satisfy the library tolerance
+|x - y| <= 1e-4 + 1e-3 |y| for unit-scale rows (rows are divided by their largest magnitude)."""
+import numpy as np
+import pytest
+import torch
+
+import longhornai_b200 as lb
+from cpu_checker import best_checker
+from gpu_util import assert_close, dev, host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def chk():
+    return best_checker()
+
+
+def rows(rng, M, K):
+    return (rng.standard_normal((M, K)) * rng.choice([1e-2, 1.0, 50.0], size=(M, 1))).astype(np.float32)
+
+
+def check(got, want, A, what):
+    scale = np.maximum(1.0, np.abs(A).max(axis=1, keepdims=True))
+    assert_close(host(got) / scale, want / scale, what=what)
+    assert lb.default_context().poll() == 0
+
+
+@pytest.mark.parametrize("M,N,K,G", [
+    (33, 256, 128, 128),        # one block of K, a second row tile's worth of padding
+    (64, 16, 256, 32),          # one 16-column strip; accumulators of 32 k
+    (257, 272, 192, 64),        # accumulators of 64 k, a last half block of K, a column tile of 16
+    (300, 528, 1024, 256),      # a group of two accumulators
+    (40, 256, 4096, 128),       # one column tile: K split over pairs
+    (520, 256 * 80, 256, 128),  # several tiles per pair
+    (48, 1040, 512, 512),
+])
+def test_int4(chk, M, N, K, G):
+    rng = np.random.default_rng(M + N + K + G)
+    A, W = rows(rng, M, K), (rng.standard_normal((K, N)) * 0.02).astype(np.float32)
+    p, s = chk.q4_quantize_groupwise(W, G)
+    C0 = rng.standard_normal((M, N)).astype(np.float32)
+    dA, dp, ds = dev(A), dev(p), dev(s)
+    check(lb.gemm_w4a16_groupwise(dA, dp, ds, G), chk.gemm_w4a16_groupwise(A, p, s, G), A, f"{M}x{N}x{K} G={G}")
+    got = lb.gemm_w4a16_groupwise(dA, dp, ds, G, C=dev(C0), alpha=0.5, beta=2.0)
+    check(got, chk.gemm_w4a16_groupwise(A, p, s, G, C0, alpha=0.5, beta=2.0), A, "alpha, beta")
+    assert torch.equal(got, lb.gemm_w4a16_groupwise(dA, dp, ds, G, C=dev(C0), alpha=0.5, beta=2.0))
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 272, 64), (130, 512, 320), (50, 128, 4096)])
+def test_int8_per_channel(chk, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    A, W = rows(rng, M, K), (rng.standard_normal((K, N)) * 0.02).astype(np.float32)
+    q, s = chk.q8_quantize_per_col(W)
+    C0 = rng.standard_normal((M, N)).astype(np.float32)
+    check(lb.gemm_w8a16_perchannel(dev(A), dev(q), dev(s)), chk.gemm_w8a16_perchannel(A, q, s), A, "int8")
+    check(lb.gemm_w8a16_perchannel(dev(A), dev(q), dev(s), C=dev(C0), alpha=0.5, beta=2.0),
+          chk.gemm_w8a16_perchannel(A, q, s, C0, alpha=0.5, beta=2.0), A, "int8 alpha, beta")
+
+
+@pytest.mark.parametrize("M,N,K,G", [(33, 272, 128, 128), (70, 528, 256, 64), (100, 64, 2048, 128)])
+def test_asymmetric_int4(M, N, K, G):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    W = torch.randn(K, N, device="cuda", generator=g) * 0.02 + 0.01
+    p, s, z = lb.q4a_quantize_groupwise(W, G)
+    A = torch.randn(M, K, device="cuda", generator=g)
+    want = (A.double() @ lb.q4a_dequantize_groupwise(p, s, z, G).double()).float()
+    check(lb.gemm_w4a16_asym(A, p, s, z, G), host(want), host(A), "asymmetric")
+
+
+def test_integers_are_exact():
+    """Small integers: every product and every partial sum is an integer below 2^24, so the result is exact."""
+    M, N, K, G = 96, 512, 512, 128
+    rng = np.random.default_rng(77)
+    q = rng.integers(-8, 8, size=(K, N)).astype(np.int64)
+    a = rng.integers(-1000, 1001, size=(M, K)).astype(np.int64)
+    packed = ((q[0::2] & 15) | ((q[1::2] & 15) << 4)).astype(np.uint8)
+    got = host(lb.gemm_w4a16_groupwise(dev(a.astype(np.float32)), dev(packed), dev(np.ones((K // G, N), np.float32)), G))
+    np.testing.assert_array_equal(got.astype(np.float64), (a @ q).astype(np.float64))
+
+
+def test_prologues_and_non_finite_rows(chk):
+    M, N, K, G = 48, 528, 512, 128
+    rng = np.random.default_rng(3)
+    W = (rng.standard_normal((K, N)) * 0.02).astype(np.float32)
+    p, s = chk.q4_quantize_groupwise(W, G)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    gamma = (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    h = chk.rmsnorm(X, gamma, 1e-5)
+    check(lb.gemm_w4a16_norm(dev(X), dev(gamma), 1e-5, dev(p), dev(s), G), chk.gemm_w4a16_groupwise(h, p, s, G), h, "norm")
+    X2 = rng.standard_normal((M, 2 * K)).astype(np.float32)
+    a = chk.swiglu(X2)
+    check(lb.gemm_w4a16_swiglu(dev(X2), dev(p), dev(s), G), chk.gemm_w4a16_groupwise(a, p, s, G), a, "swiglu")
+    bad = X.copy()
+    bad[0, 17], bad[40, 300] = np.nan, np.inf
+    got = host(lb.gemm_w4a16_groupwise(dev(bad), dev(p), dev(s), G))
+    keep = [m for m in range(M) if m not in (0, 40)]
+    assert not np.isfinite(got[[0, 40]]).any()
+    assert_close(got[keep], chk.gemm_w4a16_groupwise(X, p, s, G)[keep], what="rows without a fault")
