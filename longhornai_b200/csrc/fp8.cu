@@ -9,6 +9,7 @@
 // infinities to the largest finite value instead.
 #include "common.cuh"
 #include "dispatch.h"
+#include "quant_vec.cuh"
 
 namespace lhb {
 
@@ -47,6 +48,33 @@ __device__ __forceinline__ float e4m3_bits_to_f32(uint8_t b) {
                                : __uint_as_float((static_cast<uint32_t>(e + 120) << 23) | (static_cast<uint32_t>(m) << 20));
     return (b & 0x80u) ? -mag : mag;
 }
+
+// Vector form: the hardware conversion rounds and saturates finite values as f32_to_e4m3_bits does, except that the latter
+// has a signed zero for everything below the smallest subnormal (2^-9), where rounding to nearest would go up from
+// half of it.  Four values with a NaN or an infinity among them take the integer form.
+struct CodecFp8 {
+    static constexpr float QMAX = 448.0f;
+    static __device__ __forceinline__ uint32_t encode(float4 v) {
+        if (abs_bits_max4(v) >= 0x7f800000u)
+            return pack4(f32_to_e4m3_bits(v.x), f32_to_e4m3_bits(v.y), f32_to_e4m3_bits(v.z), f32_to_e4m3_bits(v.w));
+        auto flush = [](float x) { return fabsf(x) < 0.001953125f ? __uint_as_float(__float_as_uint(x) & 0x80000000u) : x; };
+        v = make_float4(flush(v.x), flush(v.y), flush(v.z), flush(v.w));
+        uint16_t a, b;
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(a) : "f"(v.y), "f"(v.x));
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(b) : "f"(v.w), "f"(v.z));
+        return static_cast<uint32_t>(a) | (static_cast<uint32_t>(b) << 16);
+    }
+    static __device__ __forceinline__ uint32_t mul(float4 v, float inv) {
+        return encode(make_float4(__fmul_rn(v.x, inv), __fmul_rn(v.y, inv), __fmul_rn(v.z, inv), __fmul_rn(v.w, inv)));
+    }
+    static __device__ __forceinline__ uint32_t div(float4 v, float4 s, float4) {
+        return encode(make_float4(__fdiv_rn(v.x, s.x), __fdiv_rn(v.y, s.y), __fdiv_rn(v.z, s.z), __fdiv_rn(v.w, s.w)));
+    }
+    static __device__ __forceinline__ float4 decode(uint32_t w) {
+        return make_float4(e4m3_bits_to_f32(w & 0xff), e4m3_bits_to_f32((w >> 8) & 0xff), e4m3_bits_to_f32((w >> 16) & 0xff),
+                           e4m3_bits_to_f32(w >> 24));
+    }
+};
 
 // ---- quantisers --------------------------------------------------------------------
 
@@ -187,6 +215,17 @@ int lhb_fp8_quantize_per_tensor(lhb_ctx* ctx, const float* src, uint8_t* dst, fl
     REQUIRE(n >= 0, LHB_ERR_BAD_SHAPE);
     cudaStream_t st = as_stream(stream);
     LHB_CUDA(cudaMemsetAsync(scale_out, 0, sizeof(float), st));          // doubles as the max|x| accumulator
+    if (n > 0 && vec_ok(src, dst, 1, n)) {
+        const unsigned vgrid = static_cast<unsigned>(std::min<int64_t>(ceil_div64(n, 4 * QV_THREADS), 8 * ctx->sm_count));
+        vec_absmax_kernel<<<vgrid, QV_THREADS, 0, st>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<unsigned*>(scale_out), n / 4);
+        LHB_LAUNCH_CHECK();
+        fp8_max_to_scale_kernel<<<1, 32, 0, st>>>(scale_out, 1);
+        LHB_LAUNCH_CHECK();
+        vec_quantize_tensor_kernel<CodecFp8><<<vgrid, QV_THREADS, 0, st>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<uint32_t*>(dst),
+                                                                           scale_out, n / 4);
+        LHB_LAUNCH_CHECK();
+        return LHB_OK;
+    }
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(std::max<int64_t>(1, ceil_div64(n, 1024)), 2368));
     if (n > 0) {
         fp8_absmax_kernel<<<grid, 256, 0, st>>>(src, reinterpret_cast<unsigned*>(scale_out), n);
@@ -206,6 +245,11 @@ int lhb_fp8_quantize_per_row(lhb_ctx* ctx, const float* src, uint8_t* dst, float
     REQUIRE(ctx && src && dst && scales_out, LHB_ERR_NULL);
     REQUIRE(rows >= 0 && dim > 0, LHB_ERR_BAD_SHAPE);
     if (rows == 0) return LHB_OK;
+    if (vec_ok(src, dst, 1, dim)) {
+        vec_quantize_rows_kernel<CodecFp8><<<rows, QV_THREADS, 0, as_stream(stream)>>>(src, dst, scales_out, dim);
+        LHB_LAUNCH_CHECK();
+        return LHB_OK;
+    }
     fp8_quantize_per_row_kernel<<<rows, 256, 0, as_stream(stream)>>>(src, dst, scales_out, dim);
     LHB_LAUNCH_CHECK();
     return LHB_OK;
@@ -219,14 +263,17 @@ int lhb_fp8_quantize_per_col(lhb_ctx* ctx, const float* src, uint8_t* dst, float
     LHB_CUDA(cudaMemsetAsync(scales_out, 0, sizeof(float) * static_cast<size_t>(cols), st));
     const int rpc = 128;
     dim3 grid(ceil_div(cols, 128), rows > 0 ? ceil_div(rows, rpc) : 1);
+    const bool vec = vec_ok(src, dst, rows, cols);
     if (rows > 0) {
-        fp8_col_absmax_kernel<<<grid, 128, 0, st>>>(src, reinterpret_cast<unsigned*>(scales_out), rows, cols, rpc);
+        if (vec) vec_col_absmax_kernel<<<vec_grid(rows, cols), QV_THREADS, 0, st>>>(src, reinterpret_cast<unsigned*>(scales_out), rows, cols);
+        else fp8_col_absmax_kernel<<<grid, 128, 0, st>>>(src, reinterpret_cast<unsigned*>(scales_out), rows, cols, rpc);
         LHB_LAUNCH_CHECK();
     }
     fp8_max_to_scale_kernel<<<ceil_div(cols, 256), 256, 0, st>>>(scales_out, cols);
     LHB_LAUNCH_CHECK();
     if (rows > 0) {
-        fp8_quantize_cols_kernel<<<grid, 128, 0, st>>>(src, dst, scales_out, rows, cols, rpc);
+        if (vec) vec_quantize_cols_kernel<CodecFp8><<<vec_grid(rows, cols), QV_THREADS, 0, st>>>(src, dst, scales_out, rows, cols);
+        else fp8_quantize_cols_kernel<<<grid, 128, 0, st>>>(src, dst, scales_out, rows, cols, rpc);
         LHB_LAUNCH_CHECK();
     }
     return LHB_OK;
@@ -238,6 +285,11 @@ int lhb_fp8_dequantize(lhb_ctx* ctx, const uint8_t* src, const float* scales, fl
     REQUIRE(rows >= 0 && cols > 0 && mode >= 0 && mode <= 2, LHB_ERR_BAD_SHAPE);
     const int64_t total = static_cast<int64_t>(rows) * cols;
     if (total == 0) return LHB_OK;
+    if (vec_ok(dst, src, rows, cols)) {
+        vec_dequantize_kernel<CodecFp8><<<vec_grid(rows, cols), QV_THREADS, 0, as_stream(stream)>>>(src, scales, 1.0f, dst, rows, cols, mode);
+        LHB_LAUNCH_CHECK();
+        return LHB_OK;
+    }
     fp8_dequantize_kernel<<<static_cast<unsigned>(ceil_div64(total, 256)), 256, 0, as_stream(stream)>>>(
         src, scales, dst, total, cols, mode);
     LHB_LAUNCH_CHECK();

@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "dispatch.h"
+#include "quant_vec.cuh"
 
 namespace lhb {
 
@@ -56,6 +57,84 @@ __global__ void q4a_pack_kernel(const float* __restrict__ src, const uint16_t* _
         byte |= static_cast<uint32_t>(u) << (4 * half);
     }
     packed[static_cast<int64_t>(r) * N + n] = static_cast<uint8_t>(byte);
+}
+
+// Both in one pass over the weights, vector form: as q4_quantize_vec_kernel (quant.cu), with lowest and highest weight.
+__global__ void __launch_bounds__(QV_THREADS)
+q4a_quantize_vec_kernel(const float* __restrict__ src, uint8_t* __restrict__ packed, uint16_t* __restrict__ scales_h,
+                        uint16_t* __restrict__ zeros_h, int K, int N, int G) {
+    __shared__ float4 red[2][8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = blockIdx.x * QV_COLS + 4 * lane, k0 = blockIdx.y * QV_ROWS + warp * QV_WARP_ROWS;
+    const bool ok = n < N && k0 < K;                        // K is a multiple of 16: all of a warp's rows or none
+    auto low = [](float4 a, float4 b) { return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w)); };
+    auto high = [](float4 a, float4 b) { return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w)); };
+    float4 v[QV_WARP_ROWS], lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+#pragma unroll
+    for (int i = 0; i < QV_WARP_ROWS; ++i)
+        v[i] = ok ? __ldg(reinterpret_cast<const float4*>(src + static_cast<int64_t>(k0 + i) * N + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < QV_WARP_ROWS; ++i) { lo = low(lo, v[i]); hi = high(hi, v[i]); }
+    red[0][warp][lane] = lo;
+    red[1][warp][lane] = hi;
+    __syncthreads();
+    if (!ok) return;
+    const int wpg = G / QV_WARP_ROWS, w0 = warp & ~(wpg - 1);
+    for (int w = w0; w < w0 + wpg; ++w) { lo = low(lo, red[0][w][lane]); hi = high(hi, red[1][w][lane]); }
+    auto scale_of = [](float l, float h) {
+        const float s = h2f_bits(f2h_bits(__fdiv_rn(__fsub_rn(h, l), 15.0f)));
+        return s > 0.0f ? s : 1.0f;
+    };
+    const float4 s = make_float4(scale_of(lo.x, hi.x), scale_of(lo.y, hi.y), scale_of(lo.z, hi.z), scale_of(lo.w, hi.w));
+    auto zero_of = [](float l, float sc) { return min(15, max(0, __float2int_rn(__fdiv_rn(-l, sc)))); };
+    const int4 z = make_int4(zero_of(lo.x, s.x), zero_of(lo.y, s.y), zero_of(lo.z, s.z), zero_of(lo.w, s.w));
+    if (warp == w0) {
+        const int64_t at = static_cast<int64_t>(k0 / G) * N + n;
+        *reinterpret_cast<ushort4*>(scales_h + at) = make_ushort4(f2h_bits(s.x), f2h_bits(s.y), f2h_bits(s.z), f2h_bits(s.w));
+        *reinterpret_cast<ushort4*>(zeros_h + at) = make_ushort4(f2h_bits(static_cast<float>(z.x)), f2h_bits(static_cast<float>(z.y)),
+                                                                 f2h_bits(static_cast<float>(z.z)), f2h_bits(static_cast<float>(z.w)));
+    }
+    const float4 inv = make_float4(__fdiv_rn(1.0f, s.x), __fdiv_rn(1.0f, s.y), __fdiv_rn(1.0f, s.z), __fdiv_rn(1.0f, s.w));
+    auto one = [](float x, float sc, float iv, int zz) {
+        int q;
+        if (!quick_rint(x, iv, q)) q = __float2int_rn(__fdiv_rn(x, sc));
+        return min(15, max(0, q + zz));
+    };
+    auto codes = [&](float4 x) {
+        return pack4(one(x.x, s.x, inv.x, z.x), one(x.y, s.y, inv.y, z.y), one(x.z, s.z, inv.z, z.z), one(x.w, s.w, inv.w, z.w));
+    };
+#pragma unroll
+    for (int i = 0; i < QV_WARP_ROWS; i += 2)
+        *reinterpret_cast<uint32_t*>(packed + static_cast<int64_t>((k0 + i) >> 1) * N + n) = codes(v[i]) | (codes(v[i + 1]) << 4);
+}
+
+__global__ void __launch_bounds__(QV_THREADS)
+q4a_dequantize_vec_kernel(const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales_h,
+                          const uint16_t* __restrict__ zeros_h, float* __restrict__ dst, int K, int N, int G) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = blockIdx.x * QV_COLS + 4 * lane, k0 = blockIdx.y * QV_ROWS + warp * QV_WARP_ROWS;
+    if (n >= N || k0 >= K) return;
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = __ldg(reinterpret_cast<const uint32_t*>(packed + static_cast<int64_t>((k0 >> 1) + i) * N + n));
+    const int64_t at = static_cast<int64_t>(k0 / G) * N + n;
+    const ushort4 sh = *reinterpret_cast<const ushort4*>(scales_h + at), zh = *reinterpret_cast<const ushort4*>(zeros_h + at);
+    const float4 s = make_float4(h2f_bits(sh.x), h2f_bits(sh.y), h2f_bits(sh.z), h2f_bits(sh.w));
+    const int4 z = make_int4(static_cast<int>(h2f_bits(zh.x)), static_cast<int>(h2f_bits(zh.y)), static_cast<int>(h2f_bits(zh.z)),
+                             static_cast<int>(h2f_bits(zh.w)));
+#pragma unroll
+    for (int i = 0; i < QV_WARP_ROWS; ++i) {
+        const uint32_t b = ((i & 1) ? (w[i >> 1] >> 4) : w[i >> 1]) & 0x0f0f0f0fu;
+        auto one = [&](int shift, int zz, float sc) { return __fmul_rn(static_cast<float>(static_cast<int>((b >> shift) & 15u) - zz), sc); };
+        *reinterpret_cast<float4*>(dst + static_cast<int64_t>(k0 + i) * N + n) =
+            make_float4(one(0, z.x, s.x), one(8, z.y, s.y), one(16, z.z, s.z), one(24, z.w, s.w));
+    }
+}
+
+// groups of 16, 32, 64 or 128 rows, aligned as the vector accesses need
+static bool q4a_vec_ok(const float* f32, const uint8_t* packed, const uint16_t* scales_h, const uint16_t* zeros_h, int K, int N, int G) {
+    return (G == 16 || G == 32 || G == 64 || G == 128) && vec_ok(f32, packed, K, N) &&
+           ((reinterpret_cast<uintptr_t>(scales_h) | reinterpret_cast<uintptr_t>(zeros_h)) & 7) == 0;
 }
 
 __global__ void q4a_dequantize_kernel(const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales_h,
@@ -148,6 +227,11 @@ int lhb_q4a_quantize_groupwise(lhb_ctx* ctx, const float* src, uint8_t* packed, 
     REQUIRE((K % 2) == 0 && (K % group_size) == 0, LHB_ERR_BAD_SHAPE);
     REQUIRE(K / 2 <= 65535, LHB_ERR_UNSUPPORTED);  // grid.y limit
     cudaStream_t st = as_stream(stream);
+    if (q4a_vec_ok(src, packed, scales_h, zeros_h, K, N, group_size)) {
+        q4a_quantize_vec_kernel<<<vec_grid(K, N), QV_THREADS, 0, st>>>(src, packed, scales_h, zeros_h, K, N, group_size);
+        LHB_LAUNCH_CHECK();
+        return LHB_OK;
+    }
     q4a_group_params_kernel<<<dim3(ceil_div(N, 128), K / group_size), 128, 0, st>>>(src, scales_h, zeros_h, N,
                                                                                    group_size);
     LHB_LAUNCH_CHECK();
@@ -160,6 +244,11 @@ int lhb_q4a_dequantize_groupwise(lhb_ctx* ctx, const uint8_t* packed, const uint
                                  const uint16_t* zeros_h, float* dst, int K, int N, int group_size, void* stream) {
     REQUIRE(ctx && packed && scales_h && zeros_h && dst, LHB_ERR_NULL);
     REQUIRE(K > 0 && N > 0 && group_size > 0 && (K % 2) == 0 && (K % group_size) == 0, LHB_ERR_BAD_SHAPE);
+    if (q4a_vec_ok(dst, packed, scales_h, zeros_h, K, N, group_size)) {
+        q4a_dequantize_vec_kernel<<<vec_grid(K, N), QV_THREADS, 0, as_stream(stream)>>>(packed, scales_h, zeros_h, dst, K, N, group_size);
+        LHB_LAUNCH_CHECK();
+        return LHB_OK;
+    }
     const int64_t total = static_cast<int64_t>(K) * N;
     q4a_dequantize_kernel<<<static_cast<unsigned>(ceil_div64(total, 256)), 256, 0, as_stream(stream)>>>(
         packed, scales_h, zeros_h, dst, total, N, group_size);
