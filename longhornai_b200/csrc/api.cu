@@ -162,6 +162,8 @@ int lhb_gemm_w8a16_perchannel(lhb_ctx* ctx, const float* A, const int8_t* Bq, co
         const int e = launch_wo_wide(ctx, 2, A, Bq, Bs, nullptr, C, M, N, K, 0, alpha, beta, st);
         if (e != LHB_ERR_UNSUPPORTED) return e;
     }
+    if (al && M >= knobs().wo_tc_min_m && wo_tc_ok(2, M, N, K, 0))
+        return launch_wo_tc(ctx, 2, A, Bq, Bs, nullptr, C, M, N, K, 0, alpha, beta, st);
     if (w8a16_fast_ok(M, N, K) && al)
         return launch_w8a16_fast(ctx, A, Bq, Bs, C, M, N, K, alpha, beta, st);
     return launch_w8a16_generic(A, Bq, Bs, C, M, N, K, alpha, beta, st);

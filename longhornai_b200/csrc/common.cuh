@@ -69,6 +69,7 @@ struct Knobs {
     bool pdl = true;             // LHB_PDL=0: no programmatic dependent launch
     int w4tc_min_m = 9;          // LHB_W4TC_MIN_M: fewest rows that take the W4A16 tensor-core kernel (measured: the GEMV
                                  // kernel needs 31-32 us for 9-16 rows of the 4096 x 14336 shape, this kernel 24 us)
+    int wo_tc_min_m = 9;         // LHB_WO_TC_MIN_M: fewest rows of asymmetric int4 and int8 weights for the tensor-core kernel of a few rows
     int wo_wide_min_m = 0;       // LHB_WO_WIDE_MIN_M: fewest rows that take the many-rows weight-only kernel, all formats
     bool w4tc_stream_k = false;  // LHB_W4TC_SPLIT=1: even deal of units instead of whole CTAs per column tile
     int w4tc_ctas = 0;           // LHB_W4TC_CTAS: cap on its grid

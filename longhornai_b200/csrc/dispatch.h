@@ -76,6 +76,11 @@ struct W4Peer {
 int launch_w4a16_tc(lhb_ctx* ctx, const float* A, const uint8_t* Bp, const float* Bs, float* C, int M, int N, int K,
                     int G, float alpha, float beta, cudaStream_t st, int prologue, const float* gamma, float eps,
                     const W4Peer* peer = nullptr, uint32_t* arrivals_out = nullptr);
+// the same kernel for every weight-only format (fmt as for launch_wo_wide; `peer` with int4 groups only)
+bool wo_tc_ok(int fmt, int M, int N, int K, int G);
+int launch_wo_tc(lhb_ctx* ctx, int fmt, const float* A, const void* B, const void* scales, const void* zeros, float* C, int M, int N,
+                 int K, int G, float alpha, float beta, cudaStream_t st, int prologue = 0, const float* gamma = nullptr,
+                 float eps = 0.0f, const W4Peer* peer = nullptr, uint32_t* arrivals_out = nullptr);
 // waits (bounded) until every rank's counter in this rank's arrival array has grown by `add` (peer_gather.cu)
 int launch_peer_wait(uint32_t* const* flag_table, uint32_t* state, int rank, int world, uint32_t add,
                      int timeout_ms, cudaStream_t st);

@@ -1,33 +1,31 @@
-// W4A16 group-wise GEMM for a few dozen activation rows (decode batches, small prefill
-// chunks) on the 5th-generation tensor cores.
+// Weight-only GEMMs for a few dozen activation rows (decode batches, small prefill chunks) on the
+// 5th-generation tensor cores: int4 groups, asymmetric int4 groups, int8 per channel.
 //
-// Semantics are the reference's gemm_w4a16_groupwise (src/kernels/gemm_quant.cpp:119-173;
+// Semantics of the int4 form are the reference's gemm_w4a16_groupwise (src/kernels/gemm_quant.cpp:119-173;
 // packing src/kernels/quantization.cpp:66-107): C = alpha * A * dequant(B) + beta * C with
 // A fp32 [M, K], B packed int4 [K/2, N] (low nibble = even k, two's complement) and fp32
 // scales [K/G, N].  The reference multiplies fp32 activations by fp32 dequantised weights;
-// tensor cores have no fp32 operands, so the product is rebuilt exactly from integers:
+// tensor cores have no fp32 operands, so the product is rebuilt from exact parts:
 //
-//   * every activation row is scaled by a power of two so that its maximum lies in
-//     [2^21, 2^22), rounded to an integer and split into three signed 8-bit digits
-//     (iv = 65536*d2 + 256*d1 + d0; w4tc_digits_kernel, which also applies an optional
-//     RMSNorm / SwiGLU to the row first);
-//   * converter warps expand each 128-k x 128-column tile of nibbles into int8 (16 * q: a
-//     shift and a mask per four weights) in shared memory;
-//   * kind::i8 MMAs accumulate digit x weight products in int32 in TMEM, exactly.  The MMA
-//     shape is [128 weight columns] x [3 digits * rows] x [32 k], the weights on the
-//     128-lane side so that the per-column group scale is a per-thread constant of the
-//     epilogue;
-//   * after every group of 128 k the epilogue folds
-//         acc[m] += (scale[g][n] / 16) * (65536*S2 + 256*S1 + S0)
-//     in fp32 registers (the int32 sums are below 2^22 and convert exactly) and, at the end of
-//     its K range, multiplies by the row's inverse power of two.
+//   * every activation row is scaled by a power of two so that its maximum lies in [2^14, 2^15) and
+//     split into a high and a low fp16 of 11 bits each (wo_tc_halves_kernel, which also applies an
+//     optional RMSNorm / SwiGLU to the row first);
+//   * the weights are integers of at most 8 bits (zero-point subtracted), exact in fp16: converter warps
+//     read a unit's bytes with ldmatrix.trans, turn two weights into a register with one logic and one
+//     fp16 operation, and write them to TMEM as the A operand of the MMAs (lane = weight column);
+//   * kind::f16 MMAs of [128 weight columns] x [2 halves * rows] x [16 k] add exact products in fp32 over
+//     128 k, the weights on the 128-lane side so that the per-column group scale is a per-thread constant
+//     of the epilogue;
+//   * after every 128 k the epilogue folds acc[m] += scale[g][n] * (low + high) in fp32 registers and, at
+//     the end of its K range, multiplies by the row's inverse power of two.
 //
-// The only roundings are the 22-bit activation grid (2^-22 of the row maximum), the fold
-// (three fp32 FMAs per group) and the final scale - fewer than the reference's K sequential
-// fp32 additions.  HBM traffic is the packed weights, read once.
+// HBM traffic is the weights, read once.  What bounds it: through shared memory go the raw bytes (16 KiB a
+// unit of int4) and the activation tiles (written once, read by two MMAs each); weights expanded to
+// operands in shared memory would cost three times that.  The MMA issuer is next: TMEM and shared memory
+// addresses are kept uniform (ptx::warp_index), or every instruction costs 100 cycles.
 //
 // Work is split as in the GEMV kernel: a unit is 128 k x 256 columns (16 KiB of nibbles, two
-// 128-column MMA tiles that share one digit tile); the units, ordered column tile by column
+// 128-column MMA tiles that share one activation tile); the units, ordered column tile by column
 // tile, are dealt out to one CTA per SM; a CTA that holds only part of a column tile's K
 // leaves its partial sums in scratch (same counters and scratch region as the GEMV kernel).
 // When the grid is a whole number of CTAs per column tile - the usual case: the host picks
@@ -37,11 +35,13 @@
 // one CTA per SM.  Otherwise the last CTA to arrive at a tile adds everything up alone.
 // Either way the order of the additions is fixed, so results do not vary from run to run.
 //
-// Warp roles (512 threads): 0 weight TMA producer, 1 MMA issuer, 2 TMEM allocator, 3 digit-tile
+// Warp roles (640 threads): 0 weight TMA producer, 1 MMA issuer, 2 TMEM allocator, 3 activation-tile
 // TMA producer, 4-7 and 8-11 epilogue of the first / second 128-column half (TMEM lane quarter =
-// warp % 4), 12-15 nibble -> int8 converters.
+// warp % 4), 12-15 and 16-19 converters of the first / second half.
 // Every wait is bounded (ptx::mbar_wait): a timeout sets the context's status word, the roles
 // fall through to the common exit and TMEM is freed.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cstdlib>
 
@@ -52,22 +52,25 @@
 namespace lhb {
 
 constexpr int TC_COLS = 256;                 // columns per unit
-constexpr int TC_ROWS = 64;                  // byte-rows per unit (128 k)
-constexpr int TC_RAW_BYTES = TC_COLS * TC_ROWS;          // 16 KiB
-constexpr int TC_A_BYTES = 128 * 128;                    // one 128-k x 128-column int8 operand: 16 KiB
+enum { TC_W4 = 0, TC_W4A = 1, TC_W8 = 2 };   // int4 groups, asymmetric int4 groups, int8 per channel
+__host__ __device__ constexpr int tc_rows(int fmt) { return fmt == TC_W8 ? 128 : 64; }        // byte-rows per unit (128 k)
+// a unit as it lies in memory: two boxes of 128 columns, 128-byte swizzle
+__host__ __device__ constexpr int tc_box_bytes(int fmt) { return 128 * tc_rows(fmt); }
+__host__ __device__ constexpr int tc_raw_bytes(int fmt) { return 2 * tc_box_bytes(fmt); }
 constexpr int TC_A_SLOTS = 4;                            // two units: one being multiplied, one being converted
+constexpr int TC_A_COLS = 64;                            // TMEM columns of an operand: 128 columns x 128 k of fp16
 constexpr int TC_B_STAGES = 5;
-constexpr int TC_THREADS = 512;
-constexpr int TC_CONV_WARPS = 4;
-constexpr size_t TC_DIG_BYTES = (size_t(4) << 20) - 4096;   // digit region at the head of the scratch arena
-constexpr size_t TC_SCRATCH_HEAD = size_t(4) << 20;         // its last 4 KiB: one fp32 factor per row of a pass
+constexpr int TC_THREADS = 640;
+constexpr int TC_CONV_WARPS = 4;                         // per 128-column half
+constexpr size_t TC_HALVES_BYTES = (size_t(4) << 20) - 4096;    // fp16 halves at the head of the scratch arena (more where one
+                                                                // slab's do not fit), then 4 KiB: one fp32 factor per row of a pass
 
-__host__ __device__ constexpr int tc_b_bytes(int mp) { return 3 * mp * 128; }         // [3*mp rows][128 k] int8
-__host__ __device__ constexpr int tc_raw_stages(int mp) { return mp <= 16 ? 7 : 5; }
+__host__ __device__ constexpr int tc_b_bytes(int mp) { return 2 * mp * 256; }         // [128 k / 64][2*mp rows][64 k] fp16
+__host__ __device__ constexpr int tc_raw_stages(int mp, int fmt) { return fmt == TC_W8 ? (mp <= 16 ? 5 : 4) : (mp <= 16 ? 9 : 7); }
 constexpr int TC_SC_DEPTH = 8;                           // group-scale ring: units ahead of the epilogue
-__host__ __device__ constexpr size_t tc_smem(int mp) {
-    return 1024 + size_t(TC_A_SLOTS) * TC_A_BYTES + size_t(TC_B_STAGES) * tc_b_bytes(mp) +
-           size_t(tc_raw_stages(mp)) * TC_RAW_BYTES + size_t(TC_SC_DEPTH) * TC_COLS * 4 + 512;
+__host__ __device__ constexpr size_t tc_smem(int mp, int fmt) {
+    return 1024 + size_t(TC_B_STAGES) * tc_b_bytes(mp) + size_t(tc_raw_stages(mp, fmt)) * tc_raw_bytes(fmt) +
+           size_t(TC_SC_DEPTH) * TC_COLS * 4 + 512;
 }
 
 enum { TC_PRO_NONE = 0, TC_PRO_RMSNORM = 1, TC_PRO_SWIGLU = 2 };
@@ -83,20 +86,20 @@ __device__ unsigned long long g_tc_trace[160][4][64];
 #define TC_STAMP(role, idx) do { } while (0)
 #endif
 
-// ---- activation digits ------------------------------------------------------------------
-// One CTA per row.  Output: int8 [slab][3*MP][K], row d*MP + m of a slab = digit d (0 = lowest)
-// of its row m; inv_scale[row] = the inverse of the row's power-of-two factor.
-// Rows of up to 16384 elements stay in registers between the passes.
+// ---- activation halves ------------------------------------------------------------------
+// One CTA per row.  Output: fp16 [slab][2*MP][K], row m of a slab = the high half of its row m, row MP + m the
+// low half, k in the order of the converted weights (int4: within every 16 the even k, then the odd; int8: as they are);
+// inv_scale[row] = the inverse of the row's power-of-two factor.  Rows of up to 16384 elements stay in registers between the passes.
 __global__ void __launch_bounds__(1024)
-w4tc_digits_kernel(const float* __restrict__ A, int K, int mp, int8_t* __restrict__ digits,
+wo_tc_halves_kernel(const float* __restrict__ A, int K, int mp, bool even_odd, __half* __restrict__ halves,
                    float* __restrict__ inv_scale, int prologue, const float* __restrict__ gamma, float eps) {
     __shared__ unsigned s_max[32];
     __shared__ float s_sum[32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // A comes from the kernel before; so may readers of `digits`
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // A comes from the kernel before; so may readers of `halves`
     const int row_g = blockIdx.x, slab = row_g / mp, m = row_g - slab * mp;
-    int8_t* d0_row = digits + (static_cast<int64_t>(slab) * 3 * mp + m) * K;
-    const int64_t plane = static_cast<int64_t>(mp) * K;
+    __half* hi_row = halves + (static_cast<int64_t>(slab) * 2 * mp + m) * K;
+    __half* lo_row = hi_row + static_cast<int64_t>(mp) * K;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t row_len = (prologue == TC_PRO_SWIGLU) ? 2 * static_cast<int64_t>(K) : K;
     const float* row = A + static_cast<int64_t>(row_g) * row_len;
@@ -162,30 +165,25 @@ w4tc_digits_kernel(const float* __restrict__ A, int K, int mp, int8_t* __restric
     unsigned mb = s_max[lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-    // power-of-two factor taking max|a| into [2^21, 2^22); exponent clamped
-    int se = mb ? 275 - static_cast<int>((mb >> 23) & 0xff) : 127;
+    // power-of-two factor taking max|a| into [2^14, 2^15); exponent clamped
+    int se = mb ? 268 - static_cast<int>((mb >> 23) & 0xff) : 127;
     se = max(1, min(253, se));
-    const float scl = __uint_as_float(static_cast<uint32_t>(se) << 23);
-    if (threadIdx.x == 0) inv_scale[row_g] = digit_inv_scale(mb, se);
+    const float scl = mb >= 0x7f800000u ? 0.0f : __uint_as_float(static_cast<uint32_t>(se) << 23);
+    if (threadIdx.x == 0) inv_scale[row_g] = digit_inv_scale(mb, se);        // NaN for a non-finite row
     auto put = [&](int k, float4 v) {
-        // iv = rint(v * scl) = 65536*d2 + 256*d1 + d0 with d0, d1 in [-128, 127] and |d2| <= 64: the low
-        // byte of an integer, read as signed, is its balanced digit, and what remains is divisible by 256
-        const int iv[4] = {__float2int_rn(v.x * scl), __float2int_rn(v.y * scl), __float2int_rn(v.z * scl),
-                           __float2int_rn(v.w * scl)};
-        uint32_t w0 = 0, w1 = 0, w2 = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int lo = static_cast<int>(static_cast<int8_t>(iv[j]));
-            const int iv2 = (iv[j] - lo) >> 8;
-            const int mid = static_cast<int>(static_cast<int8_t>(iv2));
-            const int hi = (iv2 - mid) >> 8;
-            w0 |= (static_cast<uint32_t>(lo) & 0xffu) << (8 * j);
-            w1 |= (static_cast<uint32_t>(mid) & 0xffu) << (8 * j);
-            w2 |= (static_cast<uint32_t>(hi) & 0xffu) << (8 * j);
+        if (scl == 0.0f) v = make_float4(0.f, 0.f, 0.f, 0.f);
+        v.x *= scl; v.y *= scl; v.z *= scl; v.w *= scl;
+        const float hx = ptx::f16_high(v.x), hy = ptx::f16_high(v.y), hz = ptx::f16_high(v.z), hw = ptx::f16_high(v.w);
+        if (!even_odd) {
+            *reinterpret_cast<uint2*>(hi_row + k) = make_uint2(ptx::pack_f16(hx, hy), ptx::pack_f16(hz, hw));
+            *reinterpret_cast<uint2*>(lo_row + k) = make_uint2(ptx::pack_f16(v.x - hx, v.y - hy), ptx::pack_f16(v.z - hz, v.w - hw));
+            return;
         }
-        *reinterpret_cast<uint32_t*>(d0_row + k) = w0;
-        *reinterpret_cast<uint32_t*>(d0_row + plane + k) = w1;
-        *reinterpret_cast<uint32_t*>(d0_row + 2 * plane + k) = w2;
+        const int at = (k & ~15) + ((k & 15) >> 1);
+        *reinterpret_cast<uint32_t*>(hi_row + at) = ptx::pack_f16(hx, hz);
+        *reinterpret_cast<uint32_t*>(hi_row + at + 8) = ptx::pack_f16(hy, hw);
+        *reinterpret_cast<uint32_t*>(lo_row + at) = ptx::pack_f16(v.x - hx, v.z - hz);
+        *reinterpret_cast<uint32_t*>(lo_row + at + 8) = ptx::pack_f16(v.y - hy, v.w - hw);
     };
     if (cached) {
 #pragma unroll
@@ -201,11 +199,12 @@ w4tc_digits_kernel(const float* __restrict__ A, int K, int mp, int8_t* __restric
 // ---- the GEMM ---------------------------------------------------------------------------
 
 struct W4TcParams {
-    const float* scales;     // [K/G, N]
+    const void* scales;      // W4: fp32 [K/G, N]; W4A: fp16 [K/G, N]; W8: fp32 [N]
+    const uint16_t* zeros;   // W4A: fp16 [K/G, N]
     float* C;                // [M, N], this slab's first row
     int M, N, K, G;          // M = rows of this slab (<= MP)
     float alpha, beta;
-    int S;                   // units per column tile = K / 128
+    int S;                   // units per column tile = K / 128, rounded up
     int units;               // column tiles * S
     int max_contrib;         // partial slots per column tile in scratch
     float* partial;          // scratch [column tile][max_contrib][M][256]
@@ -214,7 +213,7 @@ struct W4TcParams {
                              // contributors of a tile wait for each other and each adds up its share of the outputs
     int* status;
     const float* inv_scale;  // [M]
-    int dig_row0;            // first row of this slab in the digit tensor
+    int half_row0;           // first row of this slab in the halves tensor
     // Sharded use (peer_world > 0): the final values also go to columns [peer_col0, peer_col0 + N) of every
     // rank's row-major [rows, peer_ld] matrix (peer_dst[w], this slab's first row added by the kernel), and
     // the CTA that completes a column tile then adds one to counter `peer_rank` of every rank (peer_flags[w]).
@@ -233,16 +232,35 @@ __device__ __forceinline__ void tc_peer_signal(const W4TcParams& p) {
         asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(p.peer_flags[w] + p.peer_rank) : "memory");
 }
 
-// int8 x int8 -> int32 (bits 4-5 = 2; formats at bits 7-9 and 10-12 = 1), A = weights MN-major
-// (bit 15), B = digits K-major, N >> 3 at bit 17, M = 128 >> 4 at bit 24
+// fp16 x fp16 -> fp32 (bits 4-5 = 1), A in TMEM, B = activation halves K-major, N >> 3 at bit 17, M = 128 >> 4 at bit 24
 __host__ __device__ constexpr uint32_t tc_idesc(int n) {
-    return (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (static_cast<uint32_t>(n >> 3) << 17) |
-           (static_cast<uint32_t>(128 >> 4) << 24);
+    return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
 }
 
-// exact int32 -> fp32 for |v| < 2^22 without the conversion pipe
-__device__ __forceinline__ float tc_int_to_float(uint32_t v) {
-    return __uint_as_float(v + 0x4B400000u) - 12582912.0f;
+// One ldmatrix.trans register = bytes (column c, k pair r), (c + 1, r), (c, r + 1), (c + 1, r + 1).  A masked nibble in the
+// mantissa of a half under the exponent of 1024 is 1024 + u (low nibble) or 1024 + 16 u (high nibble), u = q ^ 8: one
+// logic operation and one exact fp16 operation for two weights.
+__device__ __forceinline__ uint32_t tc_sub2(uint32_t a, uint32_t b) {
+    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(a) : "r"(b));
+    return a;
+}
+__device__ __forceinline__ uint32_t tc_fma2(uint32_t a, uint32_t b, uint32_t c) {
+    asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(a) : "r"(b), "r"(c));
+    return a;
+}
+// `bias` = 1032 (W4) or 1024 + zero-point (W4A: u as it is)
+template <int FMT>
+__device__ __forceinline__ uint32_t tc_low_nibbles(uint32_t x, uint32_t bias) {
+    return tc_sub2((x & 0x000f000fu) ^ (FMT == TC_W4 ? 0x64086408u : 0x64006400u), bias);
+}
+template <int FMT>
+__device__ __forceinline__ uint32_t tc_high_nibbles(uint32_t x, uint32_t bias) {
+    return tc_fma2((x & 0x00f000f0u) ^ (FMT == TC_W4 ? 0x64806480u : 0x64006400u), 0x2c002c00u, tc_sub2(0x63806380u, bias));   // / 16 + 960 - bias
+}
+__device__ __forceinline__ void tc_ldmatrix_x4_trans(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
 }
 
 // The last contributor to a column tile adds the partial sums up and writes C.  NT threads share the
@@ -348,24 +366,25 @@ __device__ __forceinline__ void tc_sum_slice(const W4TcParams& p, const float* t
 
 __device__ __forceinline__ void tc_epi_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-template <int MP, bool PEER>
+template <int MP, bool PEER, int FMT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constant__ TensorMap tmD,
                      const W4TcParams p) {
-    constexpr int NMMA = 3 * MP;                       // MMA N: three digit rows per activation row
-    constexpr int RS = tc_raw_stages(MP);
+    constexpr int NMMA = 2 * MP;                       // MMA N: a high and a low half per activation row
+    constexpr int RS = tc_raw_stages(MP, FMT), TC_ROWS = tc_rows(FMT);
+    constexpr int TC_BOX_BYTES = tc_box_bytes(FMT), TC_RAW_BYTES = tc_raw_bytes(FMT);
     constexpr int BS = TC_B_STAGES;
     constexpr int B_BYTES = tc_b_bytes(MP);
-    constexpr int TSTRIDE = MP <= 16 ? 64 : 128;       // columns between accumulators
-    constexpr int TCOLS = 4 * TSTRIDE;                 // four accumulators of NMMA columns (two units in flight)
+    constexpr int TA = 4 * NMMA;                       // TMEM: four accumulators of NMMA columns (two units in flight), then
+    constexpr int TCOLS = 512;                         // from column TA the TC_A_SLOTS weight operands
+    static_assert(TA + TC_A_SLOTS * TC_A_COLS <= TCOLS, "TMEM columns");
     extern __shared__ uint8_t tc_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* a_ring = smem;
-    uint8_t* b_ring = a_ring + TC_A_SLOTS * TC_A_BYTES;
+    uint8_t* b_ring = smem;
     uint8_t* raw_ring = b_ring + BS * B_BYTES;
     float* sc_ring = reinterpret_cast<float*>(raw_ring + RS * TC_RAW_BYTES);       // [TC_SC_DEPTH][256]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sc_ring + TC_SC_DEPTH * TC_COLS);
-    // barriers: raw_full[RS] raw_empty[RS] a_full[3] a_empty[3] b_full[BS] b_empty[BS] t_full[4] t_empty[4]
+    // barriers: raw_full[RS] raw_empty[RS] a_full[4] a_empty[4] b_full[BS] b_empty[BS] t_full[4] t_empty[4]
     constexpr int NBARS = 2 * RS + 2 * TC_A_SLOTS + 2 * BS + 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -391,7 +410,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     const int n_units = u1 - u0;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < RS; ++s) { ptx::mbar_init(raw_full(s), 1); ptx::mbar_init(raw_empty(s), TC_CONV_WARPS); }
+        for (int s = 0; s < RS; ++s) { ptx::mbar_init(raw_full(s), 1); ptx::mbar_init(raw_empty(s), 2 * TC_CONV_WARPS); }
         for (int s = 0; s < TC_A_SLOTS; ++s) { ptx::mbar_init(a_full(s), TC_CONV_WARPS); ptx::mbar_init(a_empty(s), 1); }
         for (int s = 0; s < BS; ++s) { ptx::mbar_init(b_full(s), 1); ptx::mbar_init(b_empty(s), 1); }
         for (int s = 0; s < 4; ++s) { ptx::mbar_init(t_full(s), 1); ptx::mbar_init(t_empty(s), 128); }
@@ -407,7 +426,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
         for (int i = 0; i < first; ++i) {
             const int u = u0 + i, tile = u / S, g = u - tile * S;
             ptx::mbar_expect_tx(raw_full(i), TC_RAW_BYTES);
-            ptx::tma_load_2d(ptx::smem_u32(raw_ring + i * TC_RAW_BYTES), &tmW, tile * TC_COLS, g * TC_ROWS, raw_full(i));
+            for (int h = 0; h < 2; ++h)
+                ptx::tma_load_2d(ptx::smem_u32(raw_ring + i * TC_RAW_BYTES + h * TC_BOX_BYTES), &tmW, tile * TC_COLS + h * 128, g * TC_ROWS, raw_full(i));
         }
     }
     if (warp == 2) {
@@ -419,8 +439,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    // Digits, C, scratch, counters and the row factors belong to earlier kernels of the stream: every role
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);      // uniform, like the warp index (ptx::warp_index)
+    // Halves, C, scratch, counters and the row factors belong to earlier kernels of the stream: every role
     // that touches them waits for the programmatic dependency here.  The weight producer and the converters
     // touch only the weights and shared memory, so the first two units are converted while the previous
     // kernel drains.
@@ -436,7 +456,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                 if (!ptx::mbar_wait(raw_empty(s), ((i / RS) & 1) ^ 1, abort_flag, p.status)) break;
                 const int u = u0 + i, tile = u / S, g = u - tile * S;
                 ptx::mbar_expect_tx(raw_full(s), TC_RAW_BYTES);
-                ptx::tma_load_2d(ptx::smem_u32(raw_ring + s * TC_RAW_BYTES), &tmW, tile * TC_COLS, g * TC_ROWS, raw_full(s));
+                for (int h = 0; h < 2; ++h)
+                    ptx::tma_load_2d(ptx::smem_u32(raw_ring + s * TC_RAW_BYTES + h * TC_BOX_BYTES), &tmW, tile * TC_COLS + h * 128, g * TC_ROWS, raw_full(s));
                 issued = i + 1;
             }
             if (*abort_flag) {
@@ -449,7 +470,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             }
         }
     } else if (warp == 3) {
-        // ---- digit-tile producer: [3*MP rows][128 k] int8 per unit ----
+        // ---- activation producer: two tiles of [2*MP rows][64 k] fp16 per unit ----
         if (lane == 0) {
             int issued = 0;
             for (int i = 0; i < n_units; ++i) {
@@ -458,7 +479,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                 const int u = u0 + i, tile = u / S, g = u - tile * S;
                 const uint32_t dst = ptx::smem_u32(b_ring + s * B_BYTES);
                 ptx::mbar_expect_tx(b_full(s), B_BYTES);
-                ptx::tma_load_2d(dst, &tmD, g * 128, p.dig_row0, b_full(s));
+                ptx::tma_load_2d(dst, &tmD, g * 128, p.half_row0, b_full(s));
+                ptx::tma_load_2d(dst + B_BYTES / 2, &tmD, g * 128 + 64, p.half_row0, b_full(s));
                 issued = i + 1;
             }
             if (*abort_flag) {
@@ -470,7 +492,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: per unit, two 128-column tiles x four k32 steps ----
+        // ---- MMA issuer: per unit, two 128-column tiles x eight k16 steps ----
         if (ptx::elect_one()) {
             for (int i = 0; i < n_units; ++i) {
                 const int bs = i % BS;
@@ -486,16 +508,13 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                     if (!ptx::mbar_wait(t_empty(tb), ((n >> 2) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
                     if (i < 14 && sub == 1) TC_STAMP(3, 8 + 4 * i + 3);
                     ptx::tc_fence_after();
-                    const uint32_t sa = ptx::smem_u32(a_ring + as * TC_A_BYTES);
-                    const uint32_t d_tmem = tmem_base + tb * TSTRIDE;
+                    const uint32_t d_tmem = tmem_base + tb * NMMA, a_tmem = tmem_base + TA + as * TC_A_COLS;
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        // A: MN-major, one 128-column atom wide, 8-k atoms 1 KiB apart, 32 k per step
-                        const uint64_t da = ptx::smem_desc_sw128(sa + kk * 4096, 16, 1024);
-                        // B: K-major rows of 128 B (128 k), 8-row atoms 1 KiB apart; 32 B per step
-                        const uint64_t db = ptx::smem_desc_sw128(sb + kk * 32, 16, 1024);
-                        ptx::mma_i8_ss(d_tmem, da, db, tc_idesc(NMMA), kk != 0 ? 1u : 0u);
-                    }
+                    for (int kk = 0; kk < 8; ++kk)
+                        // B: K-major rows of 128 B (64 k), 8-row atoms 1 KiB apart; 32 B per step
+                        ptx::mma_f16_ts(d_tmem, a_tmem + 8 * kk,
+                                        ptx::smem_desc_sw128(sb + (kk >> 2) * (B_BYTES / 2) + (kk & 3) * 32, 16, 1024), tc_idesc(NMMA),
+                                        kk != 0 ? 1u : 0u);
                     ptx::tc_commit(a_empty(as));
                     ptx::tc_commit(t_full(tb));
                 }
@@ -505,43 +524,74 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             }
         }
     } else if (warp >= 12) {
-        // ---- converters: nibbles of one unit -> two int8 operand tiles ----
-        const int ct = threadIdx.x - 384;                    // 0..127
+        // ---- converters: nibbles of one unit -> two fp16 operands in TMEM.  Warp q writes lanes 32 q .. 32 q + 31 of
+        // both; lane 16 j + t holds column 32 q + 16 j + 2 (t % 8) + t / 8 of the half ----
+        const int q = warp & 3, sub = (warp - 12) >> 2, lrow = lane & 7;
+        const uint32_t a_lane = tmem_base + TA + (static_cast<uint32_t>(32 * q) << 16);
+        uint32_t ld_at[2];                                   // this lane's row of byte-rows 0 .. 31, per 16-column chunk
+#pragma unroll
+        for (int j = 0; j < 2; ++j) ld_at[j] = static_cast<uint32_t>(lane * 128 + (((2 * q + j) ^ lrow) << 4));
+        constexpr int LD = TC_ROWS / 32;                     // ldmatrix.x4 per chunk
+        // W4A: zero-points of this lane's two columns (one word), per half and chunk, a unit ahead
+        uint32_t z_next[2] = {};
+        auto fetch_zeros = [&](int i) {
+            if (FMT != TC_W4A || i >= n_units) return;
+            const int tile = (u0 + i) / S, g = ((u0 + i) - tile * S) * 128 / p.G;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int n = tile * TC_COLS + sub * 128 + 32 * q + 16 * j + 2 * (lane >> 2);
+                z_next[j] = n < p.N ? __ldg(reinterpret_cast<const uint32_t*>(p.zeros + static_cast<int64_t>(g) * p.N + n)) : 0u;
+            }
+        };
+        fetch_zeros(0);
         for (int i = 0; i < n_units; ++i) {
             const int rs = i % RS;
+            uint32_t bias[2][2];                             // chunk, column of the pair
+            if (FMT == TC_W4A) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    bias[j][0] = tc_fma2(__byte_perm(z_next[j], 0, 0x1010), 0x3c003c00u, 0x64006400u);     // 1024 + z
+                    bias[j][1] = tc_fma2(__byte_perm(z_next[j], 0, 0x3232), 0x3c003c00u, 0x64006400u);
+                }
+                fetch_zeros(i + 1);
+            }
             if (!ptx::mbar_wait(raw_full(rs), (i / RS) & 1, abort_flag, p.status)) break;
-            const uint8_t* raw = raw_ring + rs * TC_RAW_BYTES;
-            // both halves of the unit at once: eight 16-byte loads per thread in flight, one fence
-            const int as0 = (2 * i) % TC_A_SLOTS, par = (((2 * i) / TC_A_SLOTS) & 1) ^ 1;
-            if (!ptx::mbar_wait(a_empty(as0), par, abort_flag, p.status)) break;
-            if (!ptx::mbar_wait(a_empty(as0 + 1), par, abort_flag, p.status)) break;
-            uint8_t* at = a_ring + as0 * TC_A_BYTES;         // the second half's tile follows the first
-            uint4 w[8];
+            const uint32_t raw = ptx::smem_u32(raw_ring + rs * TC_RAW_BYTES);
+            const int n = 2 * i + sub, as = n % TC_A_SLOTS;
+            uint32_t x[2][4 * LD];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int task = ct + 128 * (j & 3);         // 64 byte-rows x 8 chunks of 16 columns, per half
-                w[j] = *reinterpret_cast<const uint4*>(raw + (task >> 3) * TC_COLS + (j >> 2) * 128 + (task & 7) * 16);
-            }
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int task = ct + 128 * (j & 3);
-                const int r = task >> 3, ch = task & 7;
-                // low nibbles = row k = 2r, high nibbles = row k + 1, both as 16 * q in int8
-                const uint4 ev = make_uint4((w[j].x << 4) & 0xf0f0f0f0u, (w[j].y << 4) & 0xf0f0f0f0u,
-                                            (w[j].z << 4) & 0xf0f0f0f0u, (w[j].w << 4) & 0xf0f0f0f0u);
-                const uint4 od = make_uint4(w[j].x & 0xf0f0f0f0u, w[j].y & 0xf0f0f0f0u, w[j].z & 0xf0f0f0f0u,
-                                            w[j].w & 0xf0f0f0f0u);
-                // row k of the tile: 128 B, atom k / 8, 16-byte chunk swizzled with k % 8
-                const int k = 2 * r, kin = k & 7;
-                uint8_t* base = at + (j >> 2) * TC_A_BYTES + (k >> 3) * 1024;
-                *reinterpret_cast<uint4*>(base + kin * 128 + ((ch ^ kin) << 4)) = ev;
-                *reinterpret_cast<uint4*>(base + (kin + 1) * 128 + ((ch ^ (kin + 1)) << 4)) = od;
+                for (int l = 0; l < LD; ++l) tc_ldmatrix_x4_trans(raw + sub * TC_BOX_BYTES + l * 4096 + ld_at[j], x[j] + 4 * l);
+            if (!ptx::mbar_wait(a_empty(as), ((n / TC_A_SLOTS) & 1) ^ 1, abort_flag, p.status)) break;
+            ptx::tc_fence_after();
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                uint32_t w[32];
+                if (FMT == TC_W8) {                      // 8 byte-rows = 8 k: four TMEM columns.  b ^ 0x80 under 0x64 is 1024 + 128 + b
+#pragma unroll
+                    for (int m = 0; m < 16; ++m) {
+                        const uint32_t v = x[j][m % (4 * LD)] ^ 0x80808080u;
+                        w[2 * m] = tc_sub2(__byte_perm(v, 0x64646464u, 0x4240), 0x64806480u);
+                        w[2 * m + 1] = tc_sub2(__byte_perm(v, 0x64646464u, 0x4341), 0x64806480u);
+                    }
+                } else {                                 // 8 byte-rows = 16 k: four TMEM columns of even k, four of odd
+                    const uint32_t b0 = FMT == TC_W4A ? bias[j][0] : 0x64086408u, b1 = FMT == TC_W4A ? bias[j][1] : 0x64086408u;
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        w[4 * m] = tc_low_nibbles<FMT>(x[j][m], b0);
+                        w[4 * m + 1] = tc_low_nibbles<FMT>(x[j][m] >> 8, b1);
+                        w[4 * m + 2] = tc_high_nibbles<FMT>(x[j][m], b0);
+                        w[4 * m + 3] = tc_high_nibbles<FMT>(x[j][m] >> 8, b1);
+                    }
+                }
+                ptx::tmem_st_16x64(a_lane + (static_cast<uint32_t>(16 * j) << 16) + as * TC_A_COLS, w);
             }
-            ptx::fence_proxy_async_smem();
+            ptx::tmem_st_wait();
+            ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) {
-                ptx::mbar_arrive(a_full(as0));
-                ptx::mbar_arrive(a_full(as0 + 1));
+                ptx::mbar_arrive(a_full(as));
                 ptx::mbar_arrive(raw_empty(rs));
             }
             if (threadIdx.x == 384) TC_STAMP(0, i);
@@ -550,12 +600,12 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
         // ---- epilogue: two sets of four warps, set `sub` owns the 128-column half `sub` of every unit; it
         // folds each unit's sums into fp32 registers and hands a segment over at its end ----
         const int sub = (warp - 4) >> 2, q = warp & 3;
-        const int cl = 32 * q + lane;                        // TMEM lane = column of the 128-column half
+        const int cl = 32 * q + (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1);     // TMEM lane -> column of the half
         const int et = threadIdx.x - 128;                    // 0..255
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(32 * q) << 16);
         if (et < MP) inv_s[et] = et < p.M ? p.inv_scale[et] : 0.0f;
         tc_epi_sync();
-        float acc[MP];
+        float2 acc[MP / 2];                                  // rows 2 e and 2 e + 1
         int i = 0, u = u0;
         bool alive = true;
         while (u < u1 && alive) {
@@ -563,15 +613,17 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             const int col0 = tile * TC_COLS + sub * 128;     // first column of this set's half
             const bool valid = col0 + cl < p.N;
 #pragma unroll
-            for (int m = 0; m < MP; ++m) acc[m] = 0.0f;
+            for (int m = 0; m < MP / 2; ++m) acc[m] = make_float2(0.f, 0.f);
             // Group scales: one per column and group, read from memory once per GEMM (always a DRAM
             // miss).  Every thread copies its own column's scale of the unit TC_SC_DEPTH - 1 ahead into
             // a shared-memory ring with cp.async and later reads back only what it wrote itself, so
             // the ring needs no barrier.
             float* my_sc = sc_ring + sub * 128 + cl;
             auto fetch_scale = [&](int g) {                  // one commit group per unit, even when nothing is copied
-                if (valid && g < s_end) {
-                    const float* sp = p.scales + static_cast<int64_t>((g * 128) / p.G) * p.N + col0 + cl;
+                if (FMT != TC_W8 && valid && g < s_end) {    // W4A: the word that holds this column's fp16 (N is even)
+                    const int64_t at = static_cast<int64_t>((g * 128) / p.G) * p.N + col0 + cl;
+                    const void* sp = FMT == TC_W4 ? static_cast<const void*>(static_cast<const float*>(p.scales) + at)
+                                                  : static_cast<const void*>(static_cast<const uint16_t*>(p.scales) + (at & ~int64_t(1)));
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ptx::smem_u32(my_sc + (g % TC_SC_DEPTH) * TC_COLS)),
                                  "l"(sp) : "memory");
                 }
@@ -582,17 +634,21 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             for (int g = s_begin; g < s_end; ++g, ++i) {
                 fetch_scale(g + TC_SC_DEPTH - 1);
                 asm volatile("cp.async.wait_group %0;" ::"n"(TC_SC_DEPTH - 1) : "memory");
-                const float sc = valid ? 0.0625f * my_sc[(g % TC_SC_DEPTH) * TC_COLS] : 0.0f;   // nibbles are carried as 16 * q
+                float sc = 1.0f;
+                if (FMT != TC_W8) {
+                    sc = valid ? my_sc[(g % TC_SC_DEPTH) * TC_COLS] : 0.0f;
+                    if (FMT == TC_W4A) sc = __half2float(__ushort_as_half(static_cast<uint16_t>(__float_as_uint(sc) >> (16 * (cl & 1)))));
+                }
                 const int n = 2 * i + sub, tb = n & 3;
                 if (!ptx::mbar_wait(t_full(tb), (n >> 2) & 1, abort_flag, p.status)) { alive = false; break; }
                 ptx::tc_fence_after();
-                // rows 8c..8c+7 = one 8-column slice of each digit plane; the loads of slice c + 1 are in
+                // rows 8c..8c+7 = one 8-column slice of the high and of the low halves; the loads of slice c + 1 are in
                 // flight while slice c is folded
-                const uint32_t t0 = lane_base + tb * TSTRIDE;
-                uint32_t r[2][3][8];
+                const uint32_t t0 = lane_base + tb * NMMA;
+                const float2 sc2 = make_float2(sc, sc);
+                uint32_t r[2][2][8];
                 ptx::tmem_ld_32x8(t0, r[0][0]);
                 ptx::tmem_ld_32x8(t0 + MP, r[0][1]);
-                ptx::tmem_ld_32x8(t0 + 2 * MP, r[0][2]);
 #pragma unroll
                 for (int c = 0; c < MP / 8; ++c) {
                     if (c < n_slices) {
@@ -601,18 +657,16 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                             if (c + 1 < MP / 8) {
                                 ptx::tmem_ld_32x8(t0 + 8 * (c + 1), r[(c + 1) & 1][0]);
                                 ptx::tmem_ld_32x8(t0 + MP + 8 * (c + 1), r[(c + 1) & 1][1]);
-                                ptx::tmem_ld_32x8(t0 + 2 * MP + 8 * (c + 1), r[(c + 1) & 1][2]);
                             }
                         } else {                             // last slice read: the accumulator may be overwritten
                             ptx::tc_fence_before();
                             ptx::mbar_arrive(t_empty(tb));
                         }
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const float t = fmaf(65536.0f, tc_int_to_float(r[c & 1][2][e]),
-                                                 fmaf(256.0f, tc_int_to_float(r[c & 1][1][e]),
-                                                      tc_int_to_float(r[c & 1][0][e])));
-                            acc[8 * c + e] = fmaf(sc, t, acc[8 * c + e]);
+                        for (int e = 0; e < 8; e += 2) {
+                            const float2 t = ptx::add2(make_float2(__uint_as_float(r[c & 1][0][e]), __uint_as_float(r[c & 1][0][e + 1])),
+                                                       make_float2(__uint_as_float(r[c & 1][1][e]), __uint_as_float(r[c & 1][1][e + 1])));
+                            acc[4 * c + e / 2] = FMT == TC_W8 ? ptx::add2(t, acc[4 * c + e / 2]) : ptx::fma2(t, sc2, acc[4 * c + e / 2]);
                         }
                     }
                 }
@@ -658,14 +712,19 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                 }
             };
             if (valid) {
+                const float cs = FMT == TC_W8 ? __ldg(static_cast<const float*>(p.scales) + col0 + cl) : 1.0f;
+                float val[MP];
 #pragma unroll
-                for (int m = 0; m < MP; ++m) acc[m] *= inv_s[m];
+                for (int m = 0; m < MP; ++m) {
+                    val[m] = ((m & 1) ? acc[m / 2].y : acc[m / 2].x) * inv_s[m];
+                    if (FMT == TC_W8) val[m] *= cs;
+                }
                 if (whole) {
-                    store_rows(acc);
+                    store_rows(val);
                 } else {
 #pragma unroll
                     for (int m = 0; m < MP; ++m)
-                        if (m < p.M) my_slot[m * TC_COLS] = acc[m];
+                        if (m < p.M) my_slot[m * TC_COLS] = val[m];
                 }
             }
             if (whole && TC_PW(p) > 0) {                 // the tile is complete: tell every rank
@@ -755,7 +814,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                 asm volatile("red.relaxed.gpu.global.inc.u32 [%0], %1;" ::"l"(p.counters + ft), "r"(wrap) : "memory");
             }
         } else {
-            tc_sum_partials<PEER, TC_THREADS, 5>(p, slots, ft * TC_COLS, n_contrib, threadIdx.x);
+            tc_sum_partials<PEER, TC_THREADS, 3>(p, slots, ft * TC_COLS, n_contrib, threadIdx.x);
             if (TC_PW(p) > 0) {
                 __syncthreads();
                 if (threadIdx.x == 0) tc_peer_signal(p);
@@ -768,32 +827,39 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
 // ---- host side --------------------------------------------------------------------------
 
 static int tc_slab_rows(int M) { return M > 16 ? 32 : 16; }
-static int tc_digit_rows(int mp) { return 3 * mp; }      // digit rows per slab
+static int tc_half_rows(int mp) { return 2 * mp; }       // rows of halves per slab
+// bytes of the halves of a pass: as many slabs as TC_HALVES_BYTES hold, one at least
+static size_t tc_halves_bytes(int mp, int K) { return std::max(TC_HALVES_BYTES, (static_cast<size_t>(tc_half_rows(mp)) * K * 2 + 1023) / 1024 * 1024); }
 
-bool w4a16_tc_ok(int M, int N, int K, int G) {
+bool wo_tc_ok(int fmt, int M, int N, int K, int G) {
+    if (fmt == TC_W8) {                                      // K: whole 16-byte pieces of the halves' rows
+        if (M < 1 || M > 65536 || N < 16 || (N % 16) != 0 || K < 16 || (K % 16) != 0) return false;
+        return static_cast<size_t>(tc_half_rows(tc_slab_rows(M))) * K * 2 <= (size_t(5632) << 10);
+    }
     if (M < 1 || M > 65536 || N < 16 || (N % 16) != 0 || G < 128 || (G % 128) != 0 || K < G || (K % G) != 0) return false;
-    // the digits of one slab must fit the head of the scratch arena
-    return static_cast<size_t>(tc_digit_rows(tc_slab_rows(M))) * K <= TC_DIG_BYTES;
+    return static_cast<size_t>(tc_half_rows(tc_slab_rows(M))) * K * 2 <= (size_t(5632) << 10);      // one slab's halves, in the scratch arena
 }
 
-// programmatic dependent launch between the digit pass and the GEMMs; LHB_PDL=0 turns it off
+bool w4a16_tc_ok(int M, int N, int K, int G) { return wo_tc_ok(TC_W4, M, N, K, G); }
+
+// programmatic dependent launch between the activation pass and the GEMMs; LHB_PDL=0 turns it off
 static bool tc_pdl() { return knobs().pdl; }
 
 int w4a16_tc_min_rows() { return knobs().w4tc_min_m; }
 
-template <int MP, bool PEER>
+template <int MP, bool PEER, int FMT>
 static int launch_tc_slab(lhb_ctx* ctx, const TensorMap& tmW, const TensorMap& tmD, W4TcParams p, int ctas,
                           cudaStream_t st) {
-    auto kern = gemm_w4a16_tc_kernel<MP, PEER>;
+    auto kern = gemm_w4a16_tc_kernel<MP, PEER, FMT>;
     static bool attr_set[64] = {};
     if (!attr_set[ctx->device & 63]) {
-        LHB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tc_smem(MP))));
+        LHB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tc_smem(MP, FMT))));
         attr_set[ctx->device & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, 1, 1);
     cfg.blockDim = dim3(TC_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = tc_smem(MP);
+    cfg.dynamicSmemBytes = tc_smem(MP, FMT);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -807,19 +873,25 @@ static int launch_tc_slab(lhb_ctx* ctx, const TensorMap& tmW, const TensorMap& t
 int launch_w4a16_tc(lhb_ctx* ctx, const float* A, const uint8_t* Bp, const float* Bs, float* C, int M, int N, int K,
                     int G, float alpha, float beta, cudaStream_t st, int prologue, const float* gamma, float eps,
                     const W4Peer* peer, uint32_t* arrivals_out) {
-    if (!w4a16_tc_ok(M, N, K, G)) return LHB_ERR_UNSUPPORTED;
+    return launch_wo_tc(ctx, TC_W4, A, Bp, Bs, nullptr, C, M, N, K, G, alpha, beta, st, prologue, gamma, eps, peer, arrivals_out);
+}
+
+int launch_wo_tc(lhb_ctx* ctx, int fmt, const float* A, const void* B, const void* scales, const void* zeros, float* C, int M, int N,
+                 int K, int G, float alpha, float beta, cudaStream_t st, int prologue, const float* gamma, float eps,
+                 const W4Peer* peer, uint32_t* arrivals_out) {
+    if (!wo_tc_ok(fmt, M, N, K, G) || (peer && fmt != TC_W4)) return LHB_ERR_UNSUPPORTED;
     if (arrivals_out) *arrivals_out = 0;
-    if (ctx->scratch_bytes < TC_SCRATCH_HEAD) return LHB_ERR_SCRATCH;
     TensorMap tmW;
-    if (int e = get_tensor_map_2d_u8(ctx, Bp, K / 2, N, N, TC_ROWS, TC_COLS, false, &tmW)) return e;
+    if (int e = get_tensor_map_2d_u8(ctx, B, fmt == TC_W8 ? K : K / 2, N, N, tc_rows(fmt), 128, true, &tmW)) return e;
     const int mp = tc_slab_rows(M);                         // rows per slab
-    const int drows = tc_digit_rows(mp);                    // digit rows per slab
-    const size_t slab_bytes = static_cast<size_t>(drows) * K;
-    const int slabs_per_pass = std::max<int>(1, std::min<size_t>(1024 / mp, TC_DIG_BYTES / slab_bytes));
+    const int hrows = tc_half_rows(mp);                     // rows of halves per slab
+    const size_t halves_bytes = tc_halves_bytes(mp, K), head = halves_bytes + 4096;
+    if (ctx->scratch_bytes < head) return LHB_ERR_SCRATCH;
+    const int slabs_per_pass = static_cast<int>(std::min<size_t>(1024 / mp, halves_bytes / (static_cast<size_t>(hrows) * K * 2)));
     const int rows_per_pass = slabs_per_pass * mp;
-    uint8_t* const dig = static_cast<uint8_t*>(ctx->scratch);
-    float* const inv = reinterpret_cast<float*>(dig + TC_DIG_BYTES);
-    const int S = K / 128, col_tiles = ceil_div(N, TC_COLS);
+    __half* const halves = reinterpret_cast<__half*>(ctx->scratch);
+    float* const inv = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ctx->scratch) + halves_bytes);
+    const int S = ceil_div(K, 128), col_tiles = ceil_div(N, TC_COLS);
     const int64_t units = static_cast<int64_t>(S) * col_tiles;
     if (units > (1 << 30) || col_tiles > static_cast<int>(ctx->counters_len)) return LHB_ERR_UNSUPPORTED;
     if (static_cast<int64_t>(mp) * N >= (int64_t(1) << 31)) return LHB_ERR_UNSUPPORTED;
@@ -853,41 +925,43 @@ int launch_w4a16_tc(lhb_ctx* ctx, const float* A, const uint8_t* Bp, const float
         da[0].val.programmaticStreamSerializationAllowed = 1;
         dc.attrs = da;
         dc.numAttrs = tc_pdl() ? 1 : 0;
-        LHB_CUDA(cudaLaunchKernelEx(&dc, w4tc_digits_kernel, A + pass0 * row_len, K, mp, reinterpret_cast<int8_t*>(dig),
-                                    inv, prologue, gamma, eps));
+        LHB_CUDA(cudaLaunchKernelEx(&dc, wo_tc_halves_kernel, A + pass0 * row_len, K, mp, fmt != TC_W8, halves, inv,
+                                    prologue, gamma, eps));
         const int pass_slabs = ceil_div(rows, mp);
         for (int sl = 0; sl < pass_slabs; ++sl) {
             const int m0 = pass0 + sl * mp, m = std::min(mp, M - m0);
             TensorMap tmD;
-            if (int e = get_tensor_map_2d_u8(ctx, dig, static_cast<uint64_t>(pass_slabs) * drows, K, K, drows, 128,
-                                             true, &tmD))
+            if (int e = get_tensor_map_2d_f16_sw128(ctx, halves, static_cast<uint64_t>(pass_slabs) * hrows, K,
+                                                    static_cast<uint64_t>(K) * 2, hrows, 64, &tmD))
                 return e;
             if (static_cast<size_t>(col_tiles) * max_contrib * m * TC_COLS * sizeof(float) >
-                ctx->scratch_bytes - TC_SCRATCH_HEAD)
+                ctx->scratch_bytes - head)
                 return LHB_ERR_SCRATCH;
             W4TcParams p{};
-            p.scales = Bs;
+            p.scales = scales; p.zeros = static_cast<const uint16_t*>(zeros);
             p.C = C + static_cast<int64_t>(m0) * N;
             p.M = m; p.N = N; p.K = K; p.G = G; p.alpha = alpha; p.beta = beta;
             p.S = S;
             p.units = static_cast<int>(units);
             p.max_contrib = max_contrib;
-            p.partial = reinterpret_cast<float*>(dig + TC_SCRATCH_HEAD);
+            p.partial = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ctx->scratch) + head);
             p.counters = ctx->counters;
             p.coop_sum = coop_sum;
             p.status = ctx->status_word;
             p.inv_scale = inv + (m0 - pass0);
-            p.dig_row0 = sl * drows;
+            p.half_row0 = sl * hrows;
             if (peer) {
                 p.peer_dst = reinterpret_cast<float* const*>(peer->dst_table);
                 p.peer_flags = peer->flag_table;
                 p.peer_world = peer->world; p.peer_rank = peer->rank; p.peer_ld = peer->ld; p.peer_col0 = peer->col0;
                 p.peer_row0 = m0;
             }
-            const int e = peer       ? (mp == 16 ? launch_tc_slab<16, true>(ctx, tmW, tmD, p, ctas, st)
-                                                 : launch_tc_slab<32, true>(ctx, tmW, tmD, p, ctas, st))
-                          : mp == 16 ? launch_tc_slab<16, false>(ctx, tmW, tmD, p, ctas, st)
-                                     : launch_tc_slab<32, false>(ctx, tmW, tmD, p, ctas, st);
+            const bool small = mp == 16;
+            int e;
+            if (peer) e = small ? launch_tc_slab<16, true, TC_W4>(ctx, tmW, tmD, p, ctas, st) : launch_tc_slab<32, true, TC_W4>(ctx, tmW, tmD, p, ctas, st);
+            else if (fmt == TC_W4) e = small ? launch_tc_slab<16, false, TC_W4>(ctx, tmW, tmD, p, ctas, st) : launch_tc_slab<32, false, TC_W4>(ctx, tmW, tmD, p, ctas, st);
+            else if (fmt == TC_W4A) e = small ? launch_tc_slab<16, false, TC_W4A>(ctx, tmW, tmD, p, ctas, st) : launch_tc_slab<32, false, TC_W4A>(ctx, tmW, tmD, p, ctas, st);
+            else e = small ? launch_tc_slab<16, false, TC_W8>(ctx, tmW, tmD, p, ctas, st) : launch_tc_slab<32, false, TC_W8>(ctx, tmW, tmD, p, ctas, st);
             if (e) return e;
             if (peer && arrivals_out) *arrivals_out += static_cast<uint32_t>(col_tiles);   // only launches that will signal
         }
