@@ -14,10 +14,11 @@
 // other operand, half of them fetched by each CTA.  Roles (512 threads a CTA):
 //   warps 0-7    epilogue: column = TMEM lane, warps 0-3 the first half of the rows, 4-7 the second, up to 128 fp32
 //                sums a thread; accumulators double-buffered in the 512 TMEM columns
-//   warps 8-11   converters: packed bytes -> registers (three chunks ahead) -> fp16 -> 128-byte-swizzled tile.  A
+//   warps 8-11   converters: packed bytes -> fp16 -> 128-byte-swizzled tile.  A
 //                nibble under the exponent byte 0x64 is 1024 + u; the high nibble needs no shift (1024 + 16 u, one
 //                fused multiply-add); an asymmetric weight subtracts its zero-point instead of the constant
-//   warp 12      TMA producer of the activation tiles, warp 13 MMA issuer (in the leader), warp 14 TMEM
+//   warp 12      TMA producer of the activation tiles, warp 13 MMA issuer (in the leader), warp 14 TMEM,
+//                warp 15 TMA producer of the packed weights
 // What bounds it: per k a pair spends 16 tensor cycles on 256 x 256; the shared memory of each CTA moves 120 bytes
 // a cycle for that (operand reads 1024 B, tile fills 896 B per k).  A single CTA on 128 x 256 would need 184
 // of its 128 bytes a cycle: hence the pair.  The rows per tile (a multiple of 32) are chosen so that the tiles
@@ -44,7 +45,8 @@ constexpr int WW_A_BYTES = 128 * WW_CHUNK * 2;      // this CTA's 128 columns, f
 constexpr int WW_B_BYTES = 128 * WW_CHUNK * 2;      // up to 128 rows of the high (or low) halves
 constexpr int WW_STAGE_BYTES = WW_A_BYTES + 2 * WW_B_BYTES;
 constexpr int WW_THREADS = 512;
-constexpr size_t WW_SMEM = 1024 + size_t(WW_STAGES) * WW_STAGE_BYTES + 256;
+constexpr int WW_RAW_BYTES = 24 * 1024;             // ring of packed weights: chunks of 64 k x 128 columns as they lie in memory
+constexpr size_t WW_SMEM = 1024 + size_t(WW_STAGES) * WW_STAGE_BYTES + WW_RAW_BYTES + 512;
 // Registers a thread after the split; the sum is what the launch allocates (4 x 128)
 constexpr int WW_REG_EPI = 184, WW_REG_CONV = 96, WW_REG_REST = 40;
 static_assert(2 * WW_REG_EPI + WW_REG_CONV + WW_REG_REST <= 4 * 128, "register split exceeds the launch");
@@ -52,7 +54,6 @@ static_assert(2 * WW_REG_EPI + WW_REG_CONV + WW_REG_REST <= 4 * 128, "register s
 enum { WW_W4 = 0, WW_W4A = 1, WW_W8 = 2 };
 
 struct WideParams {
-    const uint8_t* B;           // W4: packed [K/2, N]; W8: int8 [K, N]
     const void* scales;         // W4: fp32 [K/G, N]; W4A: fp16 [K/G, N]; W8: fp32 [N]
     const uint16_t* zeros;      // W4A: fp16 [K/G, N]
     float* C;                   // [M, N]
@@ -194,11 +195,15 @@ __device__ __forceinline__ void ww_nibbles(uint32_t w, uint32_t bias01, uint32_t
 
 template <int FMT>
 __global__ void __launch_bounds__(WW_THREADS, 1)
-gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constant__ TensorMap tmLo, const WideParams p) {
+gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmW, const __grid_constant__ TensorMap tmHi, const __grid_constant__ TensorMap tmLo,
+                    const WideParams p) {
+    constexpr int RROWS = FMT == WW_W8 ? WW_CHUNK : WW_CHUNK / 2;            // byte rows of a chunk
+    constexpr int RCHUNK = RROWS * 128, RS = WW_RAW_BYTES / RCHUNK;
     extern __shared__ uint8_t ww_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ww_smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WW_STAGES * WW_STAGE_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * WW_STAGES + 4);
+    uint8_t* raw_ring = smem + WW_STAGES * WW_STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(raw_ring + WW_RAW_BYTES);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * WW_STAGES + 4 + 2 * RS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_ctarank();            // 0 = leader
@@ -208,6 +213,8 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
     auto empty = [&](int s) { return bar0 + 8 * (2 * WW_STAGES + s); };          // each CTA: the stage has been multiplied
     auto t_full = [&](int b) { return bar0 + 8 * (3 * WW_STAGES + b); };         // each CTA: an accumulator is complete
     auto t_empty = [&](int b) { return bar0 + 8 * (3 * WW_STAGES + 2 + b); };    // leader: both CTAs have read it
+    auto r_full = [&](int s) { return bar0 + 8 * (3 * WW_STAGES + 4 + s); };     // each CTA: packed weights have landed
+    auto r_empty = [&](int s) { return bar0 + 8 * (3 * WW_STAGES + 4 + RS + s); };   // each CTA: they have been read
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < WW_STAGES; ++s) {
@@ -216,8 +223,10 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
             ptx::mbar_init(empty(s), 1);
         }
         for (int b = 0; b < 2; ++b) { ptx::mbar_init(t_full(b), 1); ptx::mbar_init(t_empty(b), 16); }
+        for (int s = 0; s < RS; ++s) { ptx::mbar_init(r_full(s), 1); ptx::mbar_init(r_empty(s), 4); }
         *abort_flag = 0;
         ptx::fence_mbar_init();
+        ptx::prefetch_tmap(&tmW);
         ptx::prefetch_tmap(&tmHi);
         ptx::prefetch_tmap(&tmLo);
     }
@@ -230,7 +239,7 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
     __syncthreads();
     ptx::cluster_sync_all();                                 // both CTAs' barriers exist before anyone signals them
     ptx::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);           // uniform, like the warp index
 
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int tiles = p.m_blocks * p.col_tiles, items = tiles * p.splits;
@@ -324,27 +333,10 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
         // ---- converters: 16 columns x (W4: 2 k pairs, W8: 4 k) a thread and chunk ----
         const int ct = threadIdx.x - 256, ch = ct & 7, kr = ct >> 3;      // 16-column chunk of the 128, row of 16
         constexpr int LOADS = FMT == WW_W8 ? 4 : 2;                       // rows kr, kr + 16, ... of the chunk's 64 k or 32 k pairs
-        // chunks run on across items: (item, k) of the chunk being loaded
-        int l_it = pair, l_k = pair < items ? item_k0(pair) : 0, l_k1 = pair < items ? item_k1(pair) : 0;
-        auto load = [&](uint4 (&w)[LOADS]) {
-            if (l_it >= items) return;
-            const int n = item_n(l_it) + 16 * ch;
+        auto load = [&](uint4 (&w)[LOADS], const uint8_t* raw) {
 #pragma unroll
-            for (int i = 0; i < LOADS; ++i) {
-                const int row = (FMT == WW_W8 ? l_k : l_k / 2) + kr + 16 * i;
-                const bool ok = n < p.N && (FMT == WW_W8 ? row : 2 * row) < l_k1;                    // N % 16 == 0
-                w[i] = ok ? __ldg(reinterpret_cast<const uint4*>(p.B + static_cast<int64_t>(row) * p.N + n)) : make_uint4(0, 0, 0, 0);
-            }
-            l_k += WW_CHUNK;
-            if (l_k >= l_k1) {
-                l_it += n_pairs;
-                if (l_it < items) { l_k = item_k0(l_it); l_k1 = item_k1(l_it); }
-            }
+            for (int i = 0; i < LOADS; ++i) w[i] = *reinterpret_cast<const uint4*>(raw + (kr + 16 * i) * 128 + 16 * ch);
         };
-        uint4 w[3][LOADS];                                                // the set of chunk c is c % 3: three chunks ahead
-        load(w[0]);
-        load(w[1]);
-        load(w[2]);
         uint32_t bias[8];                                                 // per column pair; W4A: of the current group
 #pragma unroll
         for (int i = 0; i < 8; ++i) bias[i] = 0x64086408u;                // 1032
@@ -353,12 +345,12 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
         const int flip = ch >> 2, c2 = (ch & 3) * 2;
         int it = pair, cc = 0;                                            // item and chunk being stored
         int k = it < items ? item_k0(it) : 0, k1 = it < items ? item_k1(it) : 0;
-        bool alive = true, fresh = true;                                  // fresh: first chunk of an item
-        while (it < items && alive) {
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-                if (it >= items) break;
-                const int s = cc % WW_STAGES;
+        bool fresh = true;                                                // first chunk of an item
+        while (it < items) {
+                const int s = cc % WW_STAGES, rs = cc % RS;
+                uint4 w[LOADS];
+                if (!ptx::mbar_wait(r_full(rs), (cc / RS) & 1, abort_flag, p.status)) break;
+                load(w, raw_ring + rs * RCHUNK);
                 if (FMT == WW_W4A && (fresh || k % p.G == 0)) {
                     const int n = item_n(it) + 16 * ch;
                     const uint16_t* zp = p.zeros + static_cast<int64_t>(k / p.G) * p.N + n;
@@ -369,7 +361,7 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
 #pragma unroll
                     for (int i = 0; i < 8; ++i) bias[i] = ww_hfma2(zz[i], 0x3c003c00u, 0x64006400u);   // 1024 + z
                 }
-                if (!ptx::mbar_wait(empty(s), ((cc / WW_STAGES) & 1) ^ 1, abort_flag, p.status)) { alive = false; break; }
+                if (!ptx::mbar_wait(empty(s), ((cc / WW_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
                 uint8_t* at = smem + s * WW_STAGE_BYTES + flip * (WW_A_BYTES / 2);
                 auto put = [&](int kk, uint4 a, uint4 b) {
                     uint8_t* base = at + kk * 128;
@@ -378,7 +370,7 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
                 };
 #pragma unroll
                 for (int i = 0; i < LOADS; ++i) {
-                    const uint4 v = w[x][i];
+                    const uint4 v = w[i];
                     const int row = kr + 16 * i;
                     if (FMT == WW_W8) {
                         uint4 a, b;
@@ -395,10 +387,12 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
                         put(2 * row + 1, make_uint4(o[0][0], o[0][1], o[1][0], o[1][1]), make_uint4(o[2][0], o[2][1], o[3][0], o[3][1]));
                     }
                 }
-                load(w[x]);
                 ptx::fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(a_full(s), 0));
+                if (lane == 0) {
+                    ptx::mbar_arrive_cluster(ptx::mapa_shared(a_full(s), 0));
+                    ptx::mbar_arrive(r_empty(rs));
+                }
                 ++cc;
                 k += WW_CHUNK;
                 fresh = k >= k1;
@@ -406,7 +400,6 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
                     it += n_pairs;
                     if (it < items) { k = item_k0(it); k1 = item_k1(it); }
                 }
-            }
         }
     } else {
         ptx::fewer_registers<WW_REG_REST>();
@@ -432,6 +425,24 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmHi, const __grid_constan
             for (int j = 0; j < WW_STAGES && ok; ++j) {
                 const int c = cc - 1 - j;
                 if (c >= 0) ok = ptx::mbar_wait(empty(c % WW_STAGES), (c / WW_STAGES) & 1, abort_flag, p.status);
+            }
+        } else if (warp == 15 && ptx::elect_one()) {
+            // ---- packed weights: they depend on nothing an earlier kernel of the stream writes ----
+            int cc = 0;
+            bool ok = true;
+            for (int it = pair; it < items && ok; it += n_pairs) {
+                const int k1 = item_k1(it), n = item_n(it);
+                for (int k = item_k0(it); k < k1; k += WW_CHUNK, ++cc) {
+                    const int s = cc % RS;
+                    if (!ptx::mbar_wait(r_empty(s), ((cc / RS) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
+                    ptx::mbar_expect_tx(r_full(s), RCHUNK);
+                    ptx::tma_load_2d(ptx::smem_u32(raw_ring + s * RCHUNK), &tmW, n, FMT == WW_W8 ? k : k / 2, r_full(s));
+                }
+            }
+            // nothing is in flight towards this CTA when it leaves
+            for (int j = 0; j < RS; ++j) {
+                const int c = cc - 1 - j;
+                if (c >= 0 && !ptx::mbar_wait(r_full(c % RS), (c / RS) & 1, abort_flag, p.status)) break;
             }
         } else if (warp == 13 && rank == 0 && ptx::elect_one()) {
             // ---- MMA issuer ----
@@ -550,7 +561,7 @@ bool wo_wide_prefer(int fmt, int M, int N, int K, int G) {
 }
 
 template <int FMT>
-static int launch_wide(lhb_ctx* ctx, const TensorMap& hi, const TensorMap& lo, const WideParams& p, cudaStream_t st) {
+static int launch_wide(lhb_ctx* ctx, const TensorMap& w, const TensorMap& hi, const TensorMap& lo, const WideParams& p, cudaStream_t st) {
     auto kern = gemm_wo_wide_kernel<FMT>;
     static bool attr_set[64] = {};
     if (!attr_set[ctx->device & 63]) {
@@ -572,7 +583,7 @@ static int launch_wide(lhb_ctx* ctx, const TensorMap& hi, const TensorMap& lo, c
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = knobs().pdl ? 2 : 1;
-    LHB_CUDA(cudaLaunchKernelEx(&cfg, kern, hi, lo, p));
+    LHB_CUDA(cudaLaunchKernelEx(&cfg, kern, w, hi, lo, p));
     return LHB_OK;
 }
 
@@ -604,18 +615,19 @@ int launch_wo_wide(lhb_ctx* ctx, int fmt, const float* A, const void* B, const v
         dc.numAttrs = knobs().pdl ? 1 : 0;
         LHB_CUDA(cudaLaunchKernelEx(&dc, wide_digits_kernel, A + m0 * row_len, K, hi, lo, inv, prologue, gamma, eps));
         const WidePlan pl = wide_plan(m, N, K, std::max(1, ctx->sm_count / 2), (ctx->scratch_bytes - used) / sizeof(float));
-        TensorMap tmHi, tmLo;
+        TensorMap tmW, tmHi, tmLo;
+        if (int e = get_tensor_map_2d_u8(ctx, B, fmt == WW_W8 ? K : K / 2, N, N, fmt == WW_W8 ? WW_CHUNK : WW_CHUNK / 2, 128, false, &tmW)) return e;
         if (int e = get_tensor_map_2d_f16_sw128(ctx, hi, m, K, static_cast<uint64_t>(K) * 2, pl.rows / 2, WW_CHUNK, &tmHi)) return e;
         if (int e = get_tensor_map_2d_f16_sw128(ctx, lo, m, K, static_cast<uint64_t>(K) * 2, pl.rows / 2, WW_CHUNK, &tmLo)) return e;
         WideParams p{};
-        p.B = static_cast<const uint8_t*>(B); p.scales = scales; p.zeros = static_cast<const uint16_t*>(zeros);
+        p.scales = scales; p.zeros = static_cast<const uint16_t*>(zeros);
         p.C = C + static_cast<int64_t>(m0) * N; p.part = part; p.inv_scale = inv;
         p.M = m; p.N = N; p.K = K; p.G = fmt == WW_W8 ? K : G;
         p.unit = fmt == WW_W8 ? 128 : std::min(G, 128);
         p.rows = pl.rows; p.m_blocks = pl.m_blocks; p.col_tiles = ceil_div(N, WW_COLS); p.splits = pl.splits;
         p.alpha = alpha; p.beta = beta; p.status = ctx->status_word;
-        const int e = fmt == WW_W4 ? launch_wide<WW_W4>(ctx, tmHi, tmLo, p, st)
-                      : fmt == WW_W4A ? launch_wide<WW_W4A>(ctx, tmHi, tmLo, p, st) : launch_wide<WW_W8>(ctx, tmHi, tmLo, p, st);
+        const int e = fmt == WW_W4 ? launch_wide<WW_W4>(ctx, tmW, tmHi, tmLo, p, st)
+                      : fmt == WW_W4A ? launch_wide<WW_W4A>(ctx, tmW, tmHi, tmLo, p, st) : launch_wide<WW_W8>(ctx, tmW, tmHi, tmLo, p, st);
         if (e) return e;
         if (pl.splits > 1) {
             const int64_t total = static_cast<int64_t>(m) * N;
