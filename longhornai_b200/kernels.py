@@ -59,14 +59,18 @@ _contexts: dict[int, Context] = {}
 
 def default_context(device: int | None = None) -> Context:
     dev = torch.cuda.current_device() if device is None else int(device)
+    c = _contexts.get(dev)
+    if c is not None:
+        return c
     with _ctx_lock:
         if dev not in _contexts:
             _contexts[dev] = Context(dev)
         return _contexts[dev]
 
 
-def _stream(device: int):
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream(device: int) -> int:
+    # the handle alone: a torch.cuda.Stream object costs ten times as much, and every call needs one
+    return torch._C._cuda_getCurrentRawStream(device)
 
 
 def _t(x: torch.Tensor, dtype, name: str) -> int:
@@ -80,7 +84,7 @@ def _t(x: torch.Tensor, dtype, name: str) -> int:
 
 
 def _ctx_for(x: torch.Tensor, ctx: Context | None) -> Context:
-    return ctx if ctx is not None else default_context(x.device.index)
+    return ctx if ctx is not None else default_context(x.get_device() if x.is_cuda else x.device.index)
 
 
 # ---------------------------------------------------------------------------
@@ -387,7 +391,7 @@ def gemm_w4a16_norm(x, gamma, eps: float, B_packed, B_scales, group_size: int, C
     M, K_ = x.shape
     N = B_packed.shape[1]
     out = _out(C, M, N, x, beta)
-    rc = c.lib.lhb_gemm_w4a16_groupwise_prologue(
+    rc = _cabi.ERR_UNSUPPORTED if 0 < M <= 2 else c.lib.lhb_gemm_w4a16_groupwise_prologue(      # one or two rows: never fused
         c.handle, _t(x, torch.float32, "x"), 1, _t(gamma, torch.float32, "gamma"), float(eps),
         _t(B_packed, torch.uint8, "B_packed"), _t(B_scales, torch.float32, "B_scales"), _t(out, torch.float32, "C"),
         M, N, K_, group_size, alpha, beta, _stream(c.device))
@@ -406,7 +410,7 @@ def gemm_w4a16_swiglu(x, B_packed, B_scales, group_size: int, C=None, alpha: flo
     K_ = K2 // 2
     N = B_packed.shape[1]
     out = _out(C, M, N, x, beta)
-    rc = c.lib.lhb_gemm_w4a16_groupwise_prologue(
+    rc = _cabi.ERR_UNSUPPORTED if 0 < M <= 2 else c.lib.lhb_gemm_w4a16_groupwise_prologue(
         c.handle, _t(x, torch.float32, "x"), 2, None, 0.0, _t(B_packed, torch.uint8, "B_packed"),
         _t(B_scales, torch.float32, "B_scales"), _t(out, torch.float32, "C"), M, N, K_, group_size, alpha, beta,
         _stream(c.device))
