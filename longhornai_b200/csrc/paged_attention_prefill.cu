@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;                            // columns: S / P buffers at 0 and 128, O buffers at 256 and 384
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);                            // columns: S / P buffers at 0 and 128, O buffers at 256 and 384
 
     if (warp < 8) {
         ptx::more_registers<PF_REG_SOFTMAX>();
