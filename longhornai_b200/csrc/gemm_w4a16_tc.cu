@@ -413,7 +413,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
         for (int s = 0; s < RS; ++s) { ptx::mbar_init(raw_full(s), 1); ptx::mbar_init(raw_empty(s), 2 * TC_CONV_WARPS); }
         for (int s = 0; s < TC_A_SLOTS; ++s) { ptx::mbar_init(a_full(s), TC_CONV_WARPS); ptx::mbar_init(a_empty(s), 1); }
         for (int s = 0; s < BS; ++s) { ptx::mbar_init(b_full(s), 1); ptx::mbar_init(b_empty(s), 1); }
-        for (int s = 0; s < 4; ++s) { ptx::mbar_init(t_full(s), 1); ptx::mbar_init(t_empty(s), 128); }
+        for (int s = 0; s < 4; ++s) { ptx::mbar_init(t_full(s), 1); ptx::mbar_init(t_empty(s), 4); }
         *abort_flag = 0;
         *epi_flag = 0;
         *final_tile = -1;
@@ -660,7 +660,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                             }
                         } else {                             // last slice read: the accumulator may be overwritten
                             ptx::tc_fence_before();
-                            ptx::mbar_arrive(t_empty(tb));
+                            ptx::mbar_arrive_warp(t_empty(tb), lane);
                         }
 #pragma unroll
                         for (int e = 0; e < 8; e += 2) {

@@ -293,7 +293,7 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmW, const __grid_constant
                         } else {                                          // the last columns are here: the accumulator may be overwritten
                             ptx::tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(t_empty(b), 0));
+                            if (lane == 0) ptx::mbar_arrive_pair(ptx::mapa_shared(t_empty(b), 0));
                         }
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
@@ -390,7 +390,7 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmW, const __grid_constant
                 ptx::fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    ptx::mbar_arrive_cluster(ptx::mapa_shared(a_full(s), 0));
+                    ptx::mbar_arrive_pair(ptx::mapa_shared(a_full(s), 0));
                     ptx::mbar_arrive(r_empty(rs));
                 }
                 ++cc;

@@ -143,12 +143,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
 
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2; ++b) {
-            ptx::mbar_init(k_full(b), 128); ptx::mbar_init(k_empty(b), 1);
-            ptx::mbar_init(v_full(b), 128); ptx::mbar_init(v_empty(b), 1);
-            ptx::mbar_init(s_full(b), 1); ptx::mbar_init(p_full(b), 256);
-            ptx::mbar_init(o_full(b), 1); ptx::mbar_init(o_free(b), 256);
+            ptx::mbar_init(k_full(b), 4); ptx::mbar_init(k_empty(b), 1);
+            ptx::mbar_init(v_full(b), 4); ptx::mbar_init(v_empty(b), 1);
+            ptx::mbar_init(s_full(b), 1); ptx::mbar_init(p_full(b), 8);
+            ptx::mbar_init(o_full(b), 1); ptx::mbar_init(o_free(b), 8);
         }
-        for (int i = 0; i < PF_PARAM_RING; ++i) ptx::mbar_init(par_full(i), 128);
+        for (int i = 0; i < PF_PARAM_RING; ++i) ptx::mbar_init(par_full(i), 4);
         *abort_flag = 0;
         *q_max = 0;
         ptx::fence_mbar_init();
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
                 ptx::tmem_ld_wait();
                 if (c0 + 32 == PF_D) {
                     ptx::tc_fence_before();
-                    ptx::mbar_arrive(o_free(b));
+                    ptx::mbar_arrive_warp(o_free(b), lane);
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
             }
             ptx::tmem_st_wait();
             ptx::tc_fence_before();
-            ptx::mbar_arrive(p_full(b));
+            ptx::mbar_arrive_warp(p_full(b), lane);
             l_a = fmaf(l_a, next_a, la.x + la.y);
             l_b = fmaf(l_b, next_b, lb.x + lb.y);
             if (j > 0 && !fold(j - 1)) { alive = false; break; }  // done long ago; this tile's PV starts meanwhile
@@ -426,15 +426,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
                 reinterpret_cast<unsigned*>(pr)[2 * PF_KEYS + cw] = vbits;
                 reinterpret_cast<unsigned*>(pr)[2 * PF_KEYS + 4 + cw] = valid;
             }
-            __syncwarp();
-            ptx::mbar_arrive(par_full(j & 3));
+            ptx::mbar_arrive_warp(par_full(j & 3), lane);
             ptx::fence_proxy_async_smem();
-            ptx::mbar_arrive(k_full(b));
+            ptx::mbar_arrive_warp(k_full(b), lane);
             if (!ptx::mbar_wait(v_empty(b), parity, abort_flag, p.status)) break;
             store(v_sm + b * PF_TILE_BYTES);
             if (j + 1 < n_tiles) load_k(j + 1);
             ptx::fence_proxy_async_smem();
-            ptx::mbar_arrive(v_full(b));
+            ptx::mbar_arrive_warp(v_full(b), lane);
         }
     } else {
         ptx::fewer_registers<PF_REG_ISSUE>();

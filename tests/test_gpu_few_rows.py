@@ -1,0 +1,57 @@
+"""GPU parity of the tensor-core kernel for a few dozen rows (weights through TMEM) at the edges of its tiles: int8 per
+channel with a K that ends inside a unit, asymmetric int4, column tiles of 16, several column tiles per CTA, K split over
+CTAs.  Outputs must satisfy the library tolerance |x - y| <= 1e-4 + 1e-3 |y| for unit-scale rows."""
+import numpy as np
+import pytest
+import torch
+
+import longhornai_b200 as lb
+from cpu_checker import best_checker
+from gpu_util import assert_close, dev, host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def chk():
+    return best_checker()
+
+
+def check(got, want, A, what):
+    scale = np.maximum(1.0, np.abs(A).max(axis=1, keepdims=True))
+    assert_close(host(got) / scale, want / scale, what=what)
+    assert lb.default_context().poll() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 16, 16), (16, 272, 144), (17, 512, 320), (32, 4096, 1024), (32, 256 * 150, 128), (12, 1040, 4112)])
+def test_int8_per_channel(chk, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    A = (rng.standard_normal((M, K)) * rng.choice([1e-2, 1.0, 50.0], size=(M, 1))).astype(np.float32)
+    W = (rng.standard_normal((K, N)) * 0.02).astype(np.float32)
+    q, s = chk.q8_quantize_per_col(W)
+    q[0, :] = -128                                          # the full range of the storage type
+    C0 = rng.standard_normal((M, N)).astype(np.float32)
+    check(lb.gemm_w8a16_perchannel(dev(A), dev(q), dev(s)), chk.gemm_w8a16_perchannel(A, q, s), A, "int8")
+    got = lb.gemm_w8a16_perchannel(dev(A), dev(q), dev(s), C=dev(C0), alpha=0.5, beta=2.0)
+    check(got, chk.gemm_w8a16_perchannel(A, q, s, C0, alpha=0.5, beta=2.0), A, "int8 alpha, beta")
+    assert torch.equal(got, lb.gemm_w8a16_perchannel(dev(A), dev(q), dev(s), C=dev(C0), alpha=0.5, beta=2.0))
+
+
+@pytest.mark.parametrize("M,N,K,G", [(9, 16, 128, 128), (17, 272, 512, 256), (32, 1040, 2048, 128), (16, 256 * 150, 128, 128)])
+def test_asymmetric_int4(M, N, K, G):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    W = torch.randn(K, N, device="cuda", generator=g) * 0.02 + 0.01
+    p, s, z = lb.q4a_quantize_groupwise(W, G)
+    A = torch.randn(M, K, device="cuda", generator=g)
+    want = (A.double() @ lb.q4a_dequantize_groupwise(p, s, z, G).double()).float()
+    check(lb.gemm_w4a16_asym(A, p, s, z, G), host(want), host(A), "asymmetric")
+
+
+def test_int8_integers_are_exact():
+    """Small integers: every product and partial sum is an integer below 2^24, so the result is exact."""
+    M, N, K = 24, 528, 448
+    rng = np.random.default_rng(5)
+    q = rng.integers(-128, 128, size=(K, N)).astype(np.int8)
+    a = rng.integers(-100, 101, size=(M, K)).astype(np.int64)
+    got = host(lb.gemm_w8a16_perchannel(dev(a.astype(np.float32)), dev(q), dev(np.ones(N, np.float32))))
+    np.testing.assert_array_equal(got.astype(np.float64), (a @ q.astype(np.int64)).astype(np.float64))
