@@ -384,8 +384,10 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     uint8_t* raw_ring = b_ring + BS * B_BYTES;
     float* sc_ring = reinterpret_cast<float*>(raw_ring + RS * TC_RAW_BYTES);       // [TC_SC_DEPTH][256]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sc_ring + TC_SC_DEPTH * TC_COLS);
-    // barriers: raw_full[RS] raw_empty[RS] a_full[4] a_empty[4] b_full[BS] b_empty[BS] t_full[4] t_empty[4]
-    constexpr int NBARS = 2 * RS + 2 * TC_A_SLOTS + 2 * BS + 8;
+    // barriers: raw_full[RS] raw_empty[RS] a_full[4] b_full[BS] b_empty[BS] t_full[4] t_empty[4].  Operand slot n % 4 is
+    // free again when accumulator n % 4 is complete: the converters wait for t_full, one commit serves both
+    constexpr int NBARS = 2 * RS + TC_A_SLOTS + 2 * BS + 8;
+    static_assert(TC_A_SLOTS == 4, "one operand slot per accumulator");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* epi_flag = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));
@@ -397,11 +399,10 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     auto raw_full = [&](int s) { return bar0 + 8 * s; };
     auto raw_empty = [&](int s) { return bar0 + 8 * (RS + s); };
     auto a_full = [&](int s) { return bar0 + 8 * (2 * RS + s); };
-    auto a_empty = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + s); };
-    auto b_full = [&](int s) { return bar0 + 8 * (2 * RS + 2 * TC_A_SLOTS + s); };
-    auto b_empty = [&](int s) { return bar0 + 8 * (2 * RS + 2 * TC_A_SLOTS + BS + s); };
-    auto t_full = [&](int s) { return bar0 + 8 * (2 * RS + 2 * TC_A_SLOTS + 2 * BS + s); };
-    auto t_empty = [&](int s) { return bar0 + 8 * (2 * RS + 2 * TC_A_SLOTS + 2 * BS + 4 + s); };
+    auto b_full = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + s); };
+    auto b_empty = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + BS + s); };
+    auto t_full = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + 2 * BS + s); };
+    auto t_empty = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + 2 * BS + 4 + s); };
 
     // this CTA's units [u0, u1), ordered column tile by column tile
     const int S = p.S;
@@ -411,7 +412,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < RS; ++s) { ptx::mbar_init(raw_full(s), 1); ptx::mbar_init(raw_empty(s), 2 * TC_CONV_WARPS); }
-        for (int s = 0; s < TC_A_SLOTS; ++s) { ptx::mbar_init(a_full(s), TC_CONV_WARPS); ptx::mbar_init(a_empty(s), 1); }
+        for (int s = 0; s < TC_A_SLOTS; ++s) { ptx::mbar_init(a_full(s), TC_CONV_WARPS); }
         for (int s = 0; s < BS; ++s) { ptx::mbar_init(b_full(s), 1); ptx::mbar_init(b_empty(s), 1); }
         for (int s = 0; s < 4; ++s) { ptx::mbar_init(t_full(s), 1); ptx::mbar_init(t_empty(s), 4); }
         *abort_flag = 0;
@@ -515,7 +516,6 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                         ptx::mma_f16_ts(d_tmem, a_tmem + 8 * kk,
                                         ptx::smem_desc_sw128(sb + (kk >> 2) * (B_BYTES / 2) + (kk & 3) * 32, 16, 1024), tc_idesc(NMMA),
                                         kk != 0 ? 1u : 0u);
-                    ptx::tc_commit(a_empty(as));
                     ptx::tc_commit(t_full(tb));
                 }
                 if (!ok) break;
@@ -563,7 +563,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int l = 0; l < LD; ++l) tc_ldmatrix_x4_trans(raw + sub * TC_BOX_BYTES + l * 4096 + ld_at[j], x[j] + 4 * l);
-            if (!ptx::mbar_wait(a_empty(as), ((n / TC_A_SLOTS) & 1) ^ 1, abort_flag, p.status)) break;
+            if (!ptx::mbar_wait(t_full(as), ((n / TC_A_SLOTS) & 1) ^ 1, abort_flag, p.status)) break;
             ptx::tc_fence_after();
 #pragma unroll
             for (int j = 0; j < 2; ++j) {

@@ -480,14 +480,12 @@ gemm_wo_wide_kernel(const __grid_constant__ TensorMap tmW, const __grid_constant
                                                      (first && pass == 0 && j == 0) ? 0u : 1u);
                             }
                         if (last) {
-                            ptx::tc_commit_pair(ptx::mapa_shared(t_full(b), 0));
-                            ptx::tc_commit_pair(ptx::mapa_shared(t_full(b), 1));
+                            ptx::tc_commit_both(t_full(b));
                             ++units;
                         }
                     }
                     if (!ok) break;
-                    ptx::tc_commit_pair(ptx::mapa_shared(empty(s), 0));   // the stage is free in both CTAs
-                    ptx::tc_commit_pair(ptx::mapa_shared(empty(s), 1));
+                    ptx::tc_commit_both(empty(s));                        // the stage is free in both CTAs
                 }
             }
         }
@@ -537,8 +535,8 @@ static WidePlan wide_plan(int M, int N, int K, int pairs, size_t part_floats) {
         for (int s = 1; s <= 16 && s <= k_blocks; ++s) {
             if (s > 1 && static_cast<size_t>(s) * M * N > part_floats) break;
             const int64_t waves = (static_cast<int64_t>(mb) * col_tiles * s + pairs - 1) / pairs;
-            const double cost = static_cast<double>(waves) * (ceil_div(k_blocks, s) * 16.0 * std::max(rows + 8, 72) + 6.0 * rows + 1500) +
-                                (s > 1 ? 6000.0 + 0.0012 * s * M * N : 0.0);
+            const double cost = static_cast<double>(waves) * (ceil_div(k_blocks, s) * (2100.0 + 5.2 * rows) + 12.0 * rows + 2500) +
+                                (s > 1 ? 5000.0 + 0.006 * s * M * N : 0.0);
             if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = WidePlan{rows, mb, s}; }
         }
     }

@@ -376,6 +376,12 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
                  : "memory");
 }
 
+// the same barrier of both CTAs (address of this CTA's) in one instruction
+__device__ __forceinline__ void tc_commit_both(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+
 // ---- register budget of a warpgroup (all of its four warps; the launch's total is never exceeded) --------------
 template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
