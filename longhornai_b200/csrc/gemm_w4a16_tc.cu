@@ -384,10 +384,10 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     uint8_t* raw_ring = b_ring + BS * B_BYTES;
     float* sc_ring = reinterpret_cast<float*>(raw_ring + RS * TC_RAW_BYTES);       // [TC_SC_DEPTH][256]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sc_ring + TC_SC_DEPTH * TC_COLS);
-    // barriers: raw_full[RS] raw_empty[RS] a_full[4] b_full[BS] b_empty[BS] t_full[4] t_empty[4].  Operand slot n % 4 is
-    // free again when accumulator n % 4 is complete: the converters wait for t_full, one commit serves both
-    constexpr int NBARS = 2 * RS + TC_A_SLOTS + 2 * BS + 8;
-    static_assert(TC_A_SLOTS == 4, "one operand slot per accumulator");
+    // barriers: raw_full[RS] raw_empty[RS] b_full[BS] b_empty[BS], then per unit slot (i % 2) a_full t_full t_empty.  Operands of
+    // a slot are free again when its accumulators are complete: the converters wait for t_full, one commit serves both
+    constexpr int NBARS = 2 * RS + 2 * BS + 6;
+    static_assert(TC_A_SLOTS == 4, "two operands (one per 128-column half) of two units");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* epi_flag = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));
@@ -398,11 +398,11 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto raw_full = [&](int s) { return bar0 + 8 * s; };
     auto raw_empty = [&](int s) { return bar0 + 8 * (RS + s); };
-    auto a_full = [&](int s) { return bar0 + 8 * (2 * RS + s); };
-    auto b_full = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + s); };
-    auto b_empty = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + BS + s); };
-    auto t_full = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + 2 * BS + s); };
-    auto t_empty = [&](int s) { return bar0 + 8 * (2 * RS + TC_A_SLOTS + 2 * BS + 4 + s); };
+    auto b_full = [&](int s) { return bar0 + 8 * (2 * RS + s); };
+    auto b_empty = [&](int s) { return bar0 + 8 * (2 * RS + BS + s); };
+    auto a_full = [&](int s) { return bar0 + 8 * (2 * RS + 2 * BS + s); };
+    auto t_full = [&](int s) { return bar0 + 8 * (2 * RS + 2 * BS + 2 + s); };
+    auto t_empty = [&](int s) { return bar0 + 8 * (2 * RS + 2 * BS + 4 + s); };
 
     // this CTA's units [u0, u1), ordered column tile by column tile
     const int S = p.S;
@@ -412,9 +412,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < RS; ++s) { ptx::mbar_init(raw_full(s), 1); ptx::mbar_init(raw_empty(s), 2 * TC_CONV_WARPS); }
-        for (int s = 0; s < TC_A_SLOTS; ++s) { ptx::mbar_init(a_full(s), TC_CONV_WARPS); }
         for (int s = 0; s < BS; ++s) { ptx::mbar_init(b_full(s), 1); ptx::mbar_init(b_empty(s), 1); }
-        for (int s = 0; s < 4; ++s) { ptx::mbar_init(t_full(s), 1); ptx::mbar_init(t_empty(s), 4); }
+        for (int s = 0; s < 2; ++s) { ptx::mbar_init(a_full(s), 2 * TC_CONV_WARPS); ptx::mbar_init(t_full(s), 1); ptx::mbar_init(t_empty(s), 8); }
         *abort_flag = 0;
         *epi_flag = 0;
         *final_tile = -1;
@@ -493,32 +492,26 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: per unit, two 128-column tiles x eight k16 steps ----
+        // ---- MMA issuer: per unit, two 128-column tiles x eight k16 steps.  Three waits and two commits a unit: with a
+        // barrier per half the issuing thread's own chain (five waits of 60-150 cycles, 1600 cycles a unit) was the limit ----
         if (ptx::elect_one()) {
             for (int i = 0; i < n_units; ++i) {
-                const int bs = i % BS;
+                const int bs = i % BS, slot = i & 1, par = (i >> 1) & 1;
+                if (!ptx::mbar_wait(t_empty(slot), par ^ 1, abort_flag, p.status)) break;
                 if (!ptx::mbar_wait(b_full(bs), (i / BS) & 1, abort_flag, p.status)) break;
-                if (i < 14) TC_STAMP(3, 8 + 4 * i);
+                if (!ptx::mbar_wait(a_full(slot), par, abort_flag, p.status)) break;
+                ptx::tc_fence_after();
                 const uint32_t sb = ptx::smem_u32(b_ring + bs * B_BYTES);
-                bool ok = true;
-#pragma unroll 1
-                for (int sub = 0; sub < 2; ++sub) {
-                    const int n = 2 * i + sub, as = n % TC_A_SLOTS, tb = n & 3;
-                    if (!ptx::mbar_wait(a_full(as), (n / TC_A_SLOTS) & 1, abort_flag, p.status)) { ok = false; break; }
-                    if (i < 14) TC_STAMP(3, 8 + 4 * i + 1 + sub);
-                    if (!ptx::mbar_wait(t_empty(tb), ((n >> 2) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
-                    if (i < 14 && sub == 1) TC_STAMP(3, 8 + 4 * i + 3);
-                    ptx::tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + tb * NMMA, a_tmem = tmem_base + TA + as * TC_A_COLS;
+                const uint32_t d_tmem = tmem_base + 2 * slot * NMMA, a_tmem = tmem_base + TA + 2 * slot * TC_A_COLS;
+#pragma unroll
+                for (int sub = 0; sub < 2; ++sub)
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
                         // B: K-major rows of 128 B (64 k), 8-row atoms 1 KiB apart; 32 B per step
-                        ptx::mma_f16_ts(d_tmem, a_tmem + 8 * kk,
+                        ptx::mma_f16_ts(d_tmem + sub * NMMA, a_tmem + sub * TC_A_COLS + 8 * kk,
                                         ptx::smem_desc_sw128(sb + (kk >> 2) * (B_BYTES / 2) + (kk & 3) * 32, 16, 1024), tc_idesc(NMMA),
                                         kk != 0 ? 1u : 0u);
-                    ptx::tc_commit(t_full(tb));
-                }
-                if (!ok) break;
+                ptx::tc_commit(t_full(slot));
                 ptx::tc_commit(b_empty(bs));
                 TC_STAMP(1, i);
             }
@@ -557,13 +550,13 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             }
             if (!ptx::mbar_wait(raw_full(rs), (i / RS) & 1, abort_flag, p.status)) break;
             const uint32_t raw = ptx::smem_u32(raw_ring + rs * TC_RAW_BYTES);
-            const int n = 2 * i + sub, as = n % TC_A_SLOTS;
+            const int slot = i & 1, as = 2 * slot + sub;
             uint32_t x[2][4 * LD];
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int l = 0; l < LD; ++l) tc_ldmatrix_x4_trans(raw + sub * TC_BOX_BYTES + l * 4096 + ld_at[j], x[j] + 4 * l);
-            if (!ptx::mbar_wait(t_full(as), ((n / TC_A_SLOTS) & 1) ^ 1, abort_flag, p.status)) break;
+            if (!ptx::mbar_wait(t_full(slot), ((i >> 1) & 1) ^ 1, abort_flag, p.status)) break;
             ptx::tc_fence_after();
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -591,7 +584,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) {
-                ptx::mbar_arrive(a_full(as));
+                ptx::mbar_arrive(a_full(slot));
                 ptx::mbar_arrive(raw_empty(rs));
             }
             if (threadIdx.x == 384) TC_STAMP(0, i);
@@ -619,18 +612,20 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
             // a shared-memory ring with cp.async and later reads back only what it wrote itself, so
             // the ring needs no barrier.
             float* my_sc = sc_ring + sub * 128 + cl;
-            auto fetch_scale = [&](int g) {                  // one commit group per unit, even when nothing is copied
+            const int upg = FMT == TC_W8 ? 1 : p.G >> 7;     // units of a group
+            int sc_unit = s_begin % upg;
+            int64_t sc_at = static_cast<int64_t>(s_begin / upg) * p.N + col0 + cl;
+            auto fetch_scale = [&](int g) {                  // consecutive units; one commit group each, even when nothing is copied
                 if (FMT != TC_W8 && valid && g < s_end) {    // W4A: the word that holds this column's fp16 (N is even)
-                    const int64_t at = static_cast<int64_t>((g * 128) / p.G) * p.N + col0 + cl;
-                    const void* sp = FMT == TC_W4 ? static_cast<const void*>(static_cast<const float*>(p.scales) + at)
-                                                  : static_cast<const void*>(static_cast<const uint16_t*>(p.scales) + (at & ~int64_t(1)));
+                    const void* sp = FMT == TC_W4 ? static_cast<const void*>(static_cast<const float*>(p.scales) + sc_at)
+                                                  : static_cast<const void*>(static_cast<const uint16_t*>(p.scales) + (sc_at & ~int64_t(1)));
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ptx::smem_u32(my_sc + (g % TC_SC_DEPTH) * TC_COLS)),
                                  "l"(sp) : "memory");
+                    if (++sc_unit == upg) { sc_unit = 0; sc_at += p.N; }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             };
             for (int j = 0; j < TC_SC_DEPTH - 1; ++j) fetch_scale(s_begin + j);
-            const int n_slices = (p.M + 7) >> 3;             // 8 rows per slice
             for (int g = s_begin; g < s_end; ++g, ++i) {
                 fetch_scale(g + TC_SC_DEPTH - 1);
                 asm volatile("cp.async.wait_group %0;" ::"n"(TC_SC_DEPTH - 1) : "memory");
@@ -639,35 +634,27 @@ gemm_w4a16_tc_kernel(const __grid_constant__ TensorMap tmW, const __grid_constan
                     sc = valid ? my_sc[(g % TC_SC_DEPTH) * TC_COLS] : 0.0f;
                     if (FMT == TC_W4A) sc = __half2float(__ushort_as_half(static_cast<uint16_t>(__float_as_uint(sc) >> (16 * (cl & 1)))));
                 }
-                const int n = 2 * i + sub, tb = n & 3;
-                if (!ptx::mbar_wait(t_full(tb), (n >> 2) & 1, abort_flag, p.status)) { alive = false; break; }
+                const int slot = i & 1;
+                if (!ptx::mbar_wait(t_full(slot), (i >> 1) & 1, abort_flag, p.status)) { alive = false; break; }
                 ptx::tc_fence_after();
-                // rows 8c..8c+7 = one 8-column slice of the high and of the low halves; the loads of slice c + 1 are in
-                // flight while slice c is folded
-                const uint32_t t0 = lane_base + tb * NMMA;
+                // 16 rows at a time: their high and low halves' sums, one wait for both
+                const uint32_t t0 = lane_base + (2 * slot + sub) * NMMA;
                 const float2 sc2 = make_float2(sc, sc);
-                uint32_t r[2][2][8];
-                ptx::tmem_ld_32x8(t0, r[0][0]);
-                ptx::tmem_ld_32x8(t0 + MP, r[0][1]);
 #pragma unroll
-                for (int c = 0; c < MP / 8; ++c) {
-                    if (c < n_slices) {
-                        ptx::tmem_ld_wait();
-                        if (c + 1 < n_slices) {
-                            if (c + 1 < MP / 8) {
-                                ptx::tmem_ld_32x8(t0 + 8 * (c + 1), r[(c + 1) & 1][0]);
-                                ptx::tmem_ld_32x8(t0 + MP + 8 * (c + 1), r[(c + 1) & 1][1]);
-                            }
-                        } else {                             // last slice read: the accumulator may be overwritten
-                            ptx::tc_fence_before();
-                            ptx::mbar_arrive_warp(t_empty(tb), lane);
-                        }
+                for (int c = 0; c < MP; c += 16) {
+                    uint32_t hi[16], lo[16];
+                    ptx::tmem_ld_32x16(t0 + c, hi);
+                    ptx::tmem_ld_32x16(t0 + MP + c, lo);
+                    ptx::tmem_ld_wait();
+                    if (c + 16 == MP) {                      // everything is read: the accumulator may be overwritten
+                        ptx::tc_fence_before();
+                        ptx::mbar_arrive_warp(t_empty(slot), lane);
+                    }
 #pragma unroll
-                        for (int e = 0; e < 8; e += 2) {
-                            const float2 t = ptx::add2(make_float2(__uint_as_float(r[c & 1][0][e]), __uint_as_float(r[c & 1][0][e + 1])),
-                                                       make_float2(__uint_as_float(r[c & 1][1][e]), __uint_as_float(r[c & 1][1][e + 1])));
-                            acc[4 * c + e / 2] = FMT == TC_W8 ? ptx::add2(t, acc[4 * c + e / 2]) : ptx::fma2(t, sc2, acc[4 * c + e / 2]);
-                        }
+                    for (int e = 0; e < 16; e += 2) {
+                        const float2 t = ptx::add2(make_float2(__uint_as_float(hi[e]), __uint_as_float(hi[e + 1])),
+                                                   make_float2(__uint_as_float(lo[e]), __uint_as_float(lo[e + 1])));
+                        acc[(c + e) / 2] = FMT == TC_W8 ? ptx::add2(t, acc[(c + e) / 2]) : ptx::fma2(t, sc2, acc[(c + e) / 2]);
                     }
                 }
                 if (et == 0) TC_STAMP(2, i);
