@@ -69,7 +69,7 @@ struct Knobs {
     bool pdl = true;             // LHB_PDL=0: no programmatic dependent launch
     int w4tc_min_m = 9;          // LHB_W4TC_MIN_M: fewest rows that take the W4A16 tensor-core kernel (measured: the GEMV
                                  // kernel needs 31-32 us for 9-16 rows of the 4096 x 14336 shape, this kernel 24 us)
-    int wo_tc_min_m = 9;         // LHB_WO_TC_MIN_M: fewest rows of asymmetric int4 and int8 weights for the tensor-core kernel of a few rows
+    int wo_tc_min_m = 0;         // LHB_WO_TC_MIN_M: fewest rows of asymmetric int4 and int8 weights for the tensor-core kernel of a few rows
     int wo_wide_min_m = 0;       // LHB_WO_WIDE_MIN_M: fewest rows that take the many-rows weight-only kernel, all formats
     bool w4tc_stream_k = false;  // LHB_W4TC_SPLIT=1: even deal of units instead of whole CTAs per column tile
     int w4tc_ctas = 0;           // LHB_W4TC_CTAS: cap on its grid
@@ -85,9 +85,45 @@ struct Knobs {
 };
 const Knobs& knobs();
 
+// Launch that may start while the kernel before it in the stream still runs (programmatic dependent launch).  The kernel
+// begins with pdl_enter(), before it touches memory: a launch on its own costs the stream one to two microseconds.
+// `early` false: an ordinary launch.  A grid of more than one CTA an SM that starts beside a GEMM piles up on the SMs which that
+// leaves first; its own spread is worth more than the launch (decode step of 4 layers, batch 32: 483 us, with the rotation
+// and append started early 494, with the attention too 522).
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl_if(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early && knobs().pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    return launch_pdl_if(true, kern, grid, block, smem, st, static_cast<A&&>(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------
+
+// Waits until everything before this kernel is complete and visible, then lets the next kernel be launched: for small
+// kernels ahead of attention, whose CTAs would otherwise take the first SMs that a GEMM leaves instead of spreading over all.
+__device__ __forceinline__ void pdl_enter_late() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Lets the next kernel of the stream be launched, then waits until everything before this one is complete and visible.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // Saturating round-half-even to [-lim, lim]; the reference's sat_round_i8 /
 // sat_round_i4 / saturate_round (src/kernels/quant.cpp:12-19, :117-124,

@@ -19,6 +19,7 @@ namespace lhb {
 __global__ void __launch_bounds__(256)
 rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ gamma, float* __restrict__ y,
                int dim, float eps) {
+    pdl_enter();
     const int64_t row = blockIdx.x;
     const float* xr = x + row * dim;
     float* yr = y + row * dim;
@@ -62,6 +63,7 @@ rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ gamma, flo
 __global__ void __launch_bounds__(256)
 rope_kernel(float* __restrict__ x, const int32_t* __restrict__ positions, int64_t n_pairs, int n_heads,
             int head_dim, float theta_base, float freq_scale, int interleaved, int pos_offset) {
+    pdl_enter_late();
     const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (idx >= n_pairs) return;
     const int half = head_dim >> 1;
@@ -88,6 +90,7 @@ rope_kernel(float* __restrict__ x, const int32_t* __restrict__ positions, int64_
 // x is [rows, 2*dim] = gate || value; y[r, i] = (gate * sigmoid(gate)) * value.
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t total, int dim) {
+    pdl_enter();
     const int64_t idx = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) * 4;
     if (idx >= total) return;
     const int64_t r = idx / dim;
@@ -126,8 +129,7 @@ int lhb_rmsnorm(lhb_ctx* ctx, const float* x, const float* gamma, float* y, int 
         REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) |
                   reinterpret_cast<uintptr_t>(y)) & 15) == 0, LHB_ERR_MISALIGNED);
     if (rows == 0) return LHB_OK;
-    rmsnorm_kernel<<<rows, 256, 0, as_stream(stream)>>>(x, gamma, y, dim, eps);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, as_stream(stream), x, gamma, y, dim, eps));
     return LHB_OK;
 }
 
@@ -138,9 +140,8 @@ static int launch_rope(float* x, const int32_t* positions, int rows, int n_heads
     REQUIRE((reinterpret_cast<uintptr_t>(x) & 7) == 0, LHB_ERR_MISALIGNED);
     const int64_t n_pairs = static_cast<int64_t>(rows) * n_heads * (head_dim / 2);
     if (n_pairs == 0) return LHB_OK;
-    rope_kernel<<<static_cast<unsigned>(ceil_div64(n_pairs, 256)), 256, 0, as_stream(stream)>>>(
-        x, positions, n_pairs, n_heads, head_dim, theta_base, freq_scale, interleaved, pos_offset);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl(rope_kernel, dim3(static_cast<unsigned>(ceil_div64(n_pairs, 256))), dim3(256), 0, as_stream(stream), x, positions,
+                        n_pairs, n_heads, head_dim, theta_base, freq_scale, interleaved, pos_offset));
     return LHB_OK;
 }
 
@@ -163,9 +164,8 @@ int lhb_swiglu(lhb_ctx* ctx, const float* x, float* y, int rows, int dim, void* 
         REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0, LHB_ERR_MISALIGNED);
     const int64_t total = static_cast<int64_t>(rows) * dim;
     if (total == 0) return LHB_OK;
-    swiglu_kernel<<<static_cast<unsigned>(ceil_div64(ceil_div64(total, 4), 256)), 256, 0, as_stream(stream)>>>(
-        x, y, total, dim);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl(swiglu_kernel, dim3(static_cast<unsigned>(ceil_div64(ceil_div64(total, 4), 256))), dim3(256), 0, as_stream(stream),
+                        x, y, total, dim));
     return LHB_OK;
 }
 

@@ -45,6 +45,7 @@ paged_kv_append_q8_kernel(int8_t* __restrict__ k_pool, int8_t* __restrict__ v_po
                           const int32_t* __restrict__ block_tables, int max_blocks,
                           const int32_t* __restrict__ past_lens, int past_len_scalar, int n_req,
                           int seq_new, lhb_paged_layout L) {
+    pdl_enter_late();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     const int64_t total = static_cast<int64_t>(n_req) * seq_new * L.n_kv_heads;
@@ -83,6 +84,7 @@ qkv_rope_append_q8_kernel(const float* __restrict__ qkv, int64_t row_stride, flo
                           const int32_t* __restrict__ positions, int n_req, int n_q_heads, lhb_paged_layout L,
                           float theta_base, float freq_scale, int interleaved) {
     __shared__ __align__(16) float rot[4][QKV_MAX_D];
+    pdl_enter_late();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int heads = n_q_heads + 2 * L.n_kv_heads;
     const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + w;
@@ -126,6 +128,7 @@ paged_kv_append_f32_kernel(float* __restrict__ k_pool, float* __restrict__ v_poo
                            const float* __restrict__ k_new, const float* __restrict__ v_new,
                            const int32_t* __restrict__ block_table, int past_len, int seq_new,
                            lhb_paged_layout L) {
+    pdl_enter_late();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (row >= static_cast<int64_t>(seq_new) * L.n_kv_heads) return;
@@ -166,11 +169,9 @@ int lhb_paged_kv_append_q8(lhb_ctx* ctx, int8_t* k_pool, int8_t* v_pool, float* 
     if (!k_new || !v_new) return LHB_ERR_NULL;
     if (past_len < 0) return LHB_ERR_BAD_SHAPE;
     const int64_t rows = static_cast<int64_t>(seq_new) * layout->n_kv_heads;
-    paged_kv_append_q8_kernel<<<static_cast<unsigned>(ceil_div64(rows, 4)), 128, 0,
-                                as_stream(stream)>>>(k_pool, v_pool, k_scales, v_scales, k_new,
-                                                     v_new, block_table, 0, nullptr, past_len, 1,
-                                                     seq_new, *layout);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl_if(ceil_div64(rows, 4) <= ctx->sm_count, paged_kv_append_q8_kernel,
+                           dim3(static_cast<unsigned>(ceil_div64(rows, 4))), dim3(128), 0, as_stream(stream),
+                        k_pool, v_pool, k_scales, v_scales, k_new, v_new, block_table, 0, nullptr, past_len, 1, seq_new, *layout));
     return LHB_OK;
 }
 
@@ -186,11 +187,9 @@ int lhb_paged_kv_append_q8_batched(lhb_ctx* ctx, int8_t* k_pool, int8_t* v_pool,
     if (seq_new <= 0 || n_requests == 0) return LHB_OK;
     if (!k_new || !v_new) return LHB_ERR_NULL;
     const int64_t rows = static_cast<int64_t>(n_requests) * seq_new * layout->n_kv_heads;
-    paged_kv_append_q8_kernel<<<static_cast<unsigned>(ceil_div64(rows, 4)), 128, 0,
-                                as_stream(stream)>>>(k_pool, v_pool, k_scales, v_scales, k_new,
-                                                     v_new, block_tables, max_blocks_per_req,
-                                                     past_lens, 0, n_requests, seq_new, *layout);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl_if(ceil_div64(rows, 4) <= ctx->sm_count, paged_kv_append_q8_kernel,
+                           dim3(static_cast<unsigned>(ceil_div64(rows, 4))), dim3(128), 0, as_stream(stream),
+                        k_pool, v_pool, k_scales, v_scales, k_new, v_new, block_tables, max_blocks_per_req, past_lens, 0, n_requests, seq_new, *layout));
     return LHB_OK;
 }
 
@@ -204,10 +203,9 @@ int lhb_paged_kv_append_f32(lhb_ctx* ctx, float* k_pool, float* v_pool, const fl
     if (!k_new || !v_new) return LHB_ERR_NULL;
     if (past_len < 0) return LHB_ERR_BAD_SHAPE;
     const int64_t rows = static_cast<int64_t>(seq_new) * layout->n_kv_heads;
-    paged_kv_append_f32_kernel<<<static_cast<unsigned>(ceil_div64(rows, 4)), 128, 0,
-                                 as_stream(stream)>>>(k_pool, v_pool, k_new, v_new, block_table,
-                                                      past_len, seq_new, *layout);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl_if(ceil_div64(rows, 4) <= ctx->sm_count, paged_kv_append_f32_kernel,
+                           dim3(static_cast<unsigned>(ceil_div64(rows, 4))), dim3(128), 0, as_stream(stream),
+                        k_pool, v_pool, k_new, v_new, block_table, past_len, seq_new, *layout));
     return LHB_OK;
 }
 
@@ -225,10 +223,9 @@ int lhb_qkv_rope_append_q8_decode(lhb_ctx* ctx, const float* qkv, int64_t row_st
     if (row_stride < static_cast<int64_t>(heads) * layout->head_dim) return LHB_ERR_BAD_SHAPE;
     if (n_requests == 0) return LHB_OK;
     const int64_t items = static_cast<int64_t>(n_requests) * heads;
-    qkv_rope_append_q8_kernel<<<static_cast<unsigned>(ceil_div64(items, 4)), 128, 0, as_stream(stream)>>>(
-        qkv, row_stride, q_out, k_pool, v_pool, k_scales, v_scales, block_tables, max_blocks_per_req, positions,
-        n_requests, n_q_heads, *layout, theta_base, freq_scale, interleaved);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl_if(ceil_div64(items, 4) <= ctx->sm_count, qkv_rope_append_q8_kernel,
+                           dim3(static_cast<unsigned>(ceil_div64(items, 4))), dim3(128), 0, as_stream(stream),
+                         qkv, row_stride, q_out, k_pool, v_pool, k_scales, v_scales, block_tables, max_blocks_per_req, positions, n_requests, n_q_heads, *layout, theta_base, freq_scale, interleaved));
     return LHB_OK;
 }
 

@@ -181,6 +181,7 @@ paged_decode_q8_kernel(const DecodeParams p) {
     constexpr float QLIM = BITS == 8 ? 4194304.0f : 1048576.0f;
     extern __shared__ __align__(128) uint8_t pd_smem[];
     __shared__ int s_last;
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int split = blockIdx.x, req = blockIdx.z;
@@ -627,8 +628,9 @@ int launch_decode_fast(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const int
         attr_set[ctx->device & 63] = true;
     }
     dim3 grid(splits, cfg.n_kv_heads * subs, n_req);
-    kern<<<grid, PD_THREADS, smem, st>>>(p);
-    LHB_LAUNCH_CHECK();
+    // early with up to one CTA an SM, or several waves (see launch_pdl_if): one request with its append 18.8 -> 13.5 us
+    const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z, slots = static_cast<int64_t>(LHB_PD_MIN_CTAS) * ctx->sm_count;
+    LHB_CUDA(launch_pdl_if(ctas <= ctx->sm_count || ctas > slots, kern, grid, dim3(PD_THREADS), smem, st, p));
     return LHB_OK;
 }
 

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) paged_decode_f32_kernel(const D
     extern __shared__ __align__(128) float df_smem[];
     __shared__ float sm_ml[DF_WARPS][DF_GROUP][2];
     __shared__ int s_last;
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tq = lane >> 3, dl = lane & 7;                  // token of a group of four, sixteenth of its row
     const int piece = blockIdx.x, req = blockIdx.z;
@@ -306,8 +307,7 @@ int launch_decode_f32_fast(lhb_ctx* ctx, const float* Q, const float* Kp, const 
         LHB_CUDA(cudaFuncSetAttribute(paged_decode_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DF_SMEM));
         attr_set[ctx->device & 63] = true;
     }
-    paged_decode_f32_kernel<<<dim3(p.pieces, p.n_kv_heads * p.subs, n_req), DF_THREADS, DF_SMEM, st>>>(p);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl(paged_decode_f32_kernel, dim3(p.pieces, p.n_kv_heads * p.subs, n_req), dim3(DF_THREADS), DF_SMEM, st, p));
     return LHB_OK;
 }
 

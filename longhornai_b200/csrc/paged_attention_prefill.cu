@@ -98,6 +98,7 @@ __device__ __forceinline__ void pf_visible(const PrefillParams& p, int pos, int 
 
 __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const PrefillParams p) {
     extern __shared__ uint8_t pf_smem_raw[];
+    pdl_enter();
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pf_smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_sm = smem;                                        // high, low operand tile
     uint8_t* k_sm = smem + 2 * PF_TILE_BYTES;                    // two tiles
@@ -488,6 +489,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) paged_prefill_q8_kernel(const P
 
 // One warp per (request, head, query): the partials of its key ranges, added in their order.
 __global__ void __launch_bounds__(256) paged_prefill_merge_kernel(const PrefillParams p) {
+    pdl_enter();
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= p.total_rows) return;
@@ -554,11 +556,9 @@ int launch_prefill_fast(lhb_ctx* ctx, const float* Q, const int8_t* Kp, const in
         LHB_CUDA(cudaFuncSetAttribute(paged_prefill_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PF_SMEM)));
         attr_set[ctx->device & 63] = true;
     }
-    paged_prefill_q8_kernel<<<dim3(p.row_tiles * p.splits, p.n_kv_heads, n_req), PF_THREADS, PF_SMEM, st>>>(p);
-    LHB_LAUNCH_CHECK();
+    LHB_CUDA(launch_pdl(paged_prefill_q8_kernel, dim3(p.row_tiles * p.splits, p.n_kv_heads, n_req), dim3(PF_THREADS), PF_SMEM, st, p));
     if (p.splits > 1) {
-        paged_prefill_merge_kernel<<<static_cast<unsigned>(ceil_div64(p.total_rows, 8)), 256, 0, st>>>(p);
-        LHB_LAUNCH_CHECK();
+        LHB_CUDA(launch_pdl(paged_prefill_merge_kernel, dim3(static_cast<unsigned>(ceil_div64(p.total_rows, 8))), dim3(256), 0, st, p));
     }
     return LHB_OK;
 }
