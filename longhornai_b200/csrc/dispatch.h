@@ -31,6 +31,7 @@ int launch_w8a16_fast(lhb_ctx* ctx, const float* A, const int8_t* Bq, const floa
 
 // tcgen05 W8A8 (gemm_w8a8_tc.cu)
 bool w8a8_fast_ok(int M, int N, int K);
+bool w8a8_tc_ok(int M, int N, int K);      // the same without its fewest rows
 int launch_w8a8_fast(lhb_ctx* ctx, const int8_t* Aq, const int8_t* Bq, const float* as,
                      const float* bs, float* C, int M, int N, int K, float alpha, float beta,
                      cudaStream_t st);

@@ -306,7 +306,7 @@ int lhb_gemm_fp8_e4m3(lhb_ctx* ctx, const uint8_t* A, const uint8_t* B, float A_
     const float combined = alpha * A_scale * B_scale;       // the reference's order (gemm_quant.cpp:91)
     cudaStream_t st = as_stream(stream);
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (w8a8_fast_ok(M, N, K) && al16(A) && al16(B) && al16(C))
+    if ((beta == 0.0f ? w8a8_tc_ok(M, N, K) : w8a8_fast_ok(M, N, K)) && al16(A) && al16(B) && al16(C))
         return launch_fp8_fast(ctx, A, B, combined, C, M, N, K, beta, st);
     return launch_fp8_generic(A, B, combined, C, M, N, K, beta, st);
 }

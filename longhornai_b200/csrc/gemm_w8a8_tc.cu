@@ -71,6 +71,7 @@ struct W8Params {
     int M, N, K;
     float alpha, beta;
     int tiles_m, tiles_n;
+    int splits;            // parts of K (1 = whole), single-CTA kernel with beta 0 only
     int* status;
     float combined;        // fp8: alpha * A_scale * B_scale (a_scales / b_scales unused)
 };
@@ -113,6 +114,22 @@ __device__ __forceinline__ void f8_store_chunk(int64_t row_off, int nb, const ui
     }
 }
 
+// The same for a part of a split K (beta 0): this thread's earlier parts wait in C, the last part scales.
+__device__ __forceinline__ void f8_add_chunk(int64_t row_off, int nb, const uint32_t (&r)[32], bool first, bool last, const W8Params& p) {
+    float* crow = p.C + row_off + nb;
+    const int cols = min(32, p.N - nb);                    // a multiple of 16
+    float4 old[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) old[j] = !first && 4 * j < cols ? *reinterpret_cast<const float4*>(crow + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (4 * j >= cols) break;
+        float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+        if (!first) { v.x = __fadd_rn(old[j].x, v.x); v.y = __fadd_rn(old[j].y, v.y); v.z = __fadd_rn(old[j].z, v.z); v.w = __fadd_rn(old[j].w, v.w); }
+        if (last) { v.x = __fmul_rn(p.combined, v.x); v.y = __fmul_rn(p.combined, v.y); v.z = __fmul_rn(p.combined, v.z); v.w = __fmul_rn(p.combined, v.w); }
+        *reinterpret_cast<float4*>(crow + 4 * j) = v;
+    }
+}
 
 // Tile index -> (row block, column block).  Row blocks run fastest for a plain call (consecutive
 // CTAs share a weight tile in L2).  The N-sharded call runs column blocks fastest: its epilogues
@@ -152,6 +169,37 @@ __device__ __forceinline__ void w8_push_chunk(float4* stg, int lane, int row0, i
         }
     }
     __syncwarp();                                         // the tile is free for the next chunk
+}
+
+// A chunk of a split K: the integer sums are added to C's words, which hold integers until w8_finish_kernel scales them.
+// Integer sums do not depend on their order.  Staged as above, so that an instruction adds to 128 bytes of one row.
+__device__ __forceinline__ void w8_add_chunk(float4* stg, int lane, int row0, int nb, const uint32_t (&r)[32], const W8Params& p) {
+#pragma unroll
+    for (int j4 = 0; j4 < 8; ++j4)
+        reinterpret_cast<uint4*>(stg)[lane * 8 + (j4 ^ (lane & 7))] = make_uint4(r[4 * j4], r[4 * j4 + 1], r[4 * j4 + 2], r[4 * j4 + 3]);
+    __syncwarp();
+    const int rows = min(32, p.M - row0);
+    if (nb + lane < p.N)
+        for (int rr = 0; rr < rows; ++rr) {
+            const int v = reinterpret_cast<const int*>(stg)[(rr * 8 + ((lane >> 2) ^ (rr & 7))) * 4 + (lane & 3)];
+            atomicAdd(reinterpret_cast<int*>(p.C) + static_cast<int64_t>(row0 + rr) * p.N + nb + lane, v);
+        }
+    __syncwarp();                                         // the tile is free for the next chunk
+}
+
+// C in place: integer sums -> ((alpha*a_s)*b_s[n])*float(acc), four columns a thread
+__global__ void __launch_bounds__(256)
+w8_finish_kernel(float* __restrict__ C, const float* __restrict__ a_scales, const float* __restrict__ b_scales, float alpha, int64_t total4, int n4) {
+    pdl_enter();
+    const int64_t i = blockIdx.x * static_cast<int64_t>(256) + threadIdx.x;
+    if (i >= total4) return;
+    const int m = static_cast<int>(i / n4), n = static_cast<int>(i - static_cast<int64_t>(m) * n4);
+    const int4 v = reinterpret_cast<const int4*>(C)[i];
+    const float sa = __fmul_rn(alpha, a_scales[m]);
+    const float4 bs = reinterpret_cast<const float4*>(b_scales)[n];
+    reinterpret_cast<float4*>(C)[i] =
+        make_float4(__fmul_rn(__fmul_rn(sa, bs.x), static_cast<float>(v.x)), __fmul_rn(__fmul_rn(sa, bs.y), static_cast<float>(v.y)),
+                    __fmul_rn(__fmul_rn(sa, bs.z), static_cast<float>(v.z)), __fmul_rn(__fmul_rn(sa, bs.w), static_cast<float>(v.w)));
 }
 
 // The bulk-store form of the same push: the staged chunk (the XOR pattern above is exactly the TMA
@@ -261,17 +309,32 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // The i-th item of this CTA -> tile and its part of K (one part unless K is split).  int8: the parts of a tile go to
+    // different CTAs; fp8: to the same one, one after the other
     const int n_tiles = p.tiles_m * p.tiles_n;
+    auto next_item = [&](int i, int& tile, int& part) {
+        if (F8) {
+            tile = static_cast<int>(blockIdx.x) + i / p.splits * static_cast<int>(gridDim.x);
+            part = i % p.splits;
+            return tile < n_tiles;
+        }
+        const int item = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
+        part = item / n_tiles;
+        tile = item - part * n_tiles;
+        return item < n_tiles * p.splits;
+    };
     const int num_kb = (p.K + W8_BK - 1) / W8_BK;
+    auto kb_from = [&](int part) { return static_cast<int>(static_cast<int64_t>(num_kb) * part / p.splits); };
 
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0;
-            for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x) {
+            int it = 0, tile, part;
+            for (int ti = 0; next_item(ti, tile, part) && !*abort_flag; ++ti) {
                 int mb_, nb_;
+                const int kb1 = kb_from(part + 1);
                 w8_tile_blocks(tile, p.tiles_m, p.tiles_n, p.n_dst > 1, mb_, nb_);
                 const int m0 = mb_ * W8_BM, n0 = nb_ * W8_BN;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                for (int kb = kb_from(part); kb < kb1; ++kb, ++it) {
                     const int s = it % W8_STAGES;
                     if (!ptx::mbar_wait(empty_bar(s), ((it / W8_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
                     ptx::mbar_expect_tx(full_bar(s), W8_STAGE_BYTES);
@@ -293,14 +356,14 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
         }
     } else if (warp == 1) {
         if (ptx::elect_one()) {
-            int it = 0, ti = 0;
-            for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x, ++ti) {
-                const int buf = ti & 1;
+            int it = 0, tile, part;
+            for (int ti = 0; next_item(ti, tile, part) && !*abort_flag; ++ti) {
+                const int buf = ti & 1, kb0 = kb_from(part), kb1 = kb_from(part + 1);
                 if (!ptx::mbar_wait(tempty_bar(buf), ((ti >> 1) & 1) ^ 1, abort_flag, p.status)) break;
                 ptx::tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * W8_BN;
                 bool ok = true;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % W8_STAGES;
                     if (!ptx::mbar_wait(full_bar(s), (it / W8_STAGES) & 1, abort_flag, p.status)) { ok = false; break; }
                     ptx::tc_fence_after();
@@ -313,8 +376,8 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
                         // B: MN-major, 128 columns per atom row, 8 k-rows = 1024 B, the second
                         // 128-column box lies W8_BK*128 bytes further; K advances 32 rows
                         const uint64_t db = ptx::smem_desc_sw128(sb + k4 * 32 * 128, W8_BK * 128, 1024);
-                        if (F8) ptx::mma_f8_ss(d_tmem, da, db, f8_idesc(W8_BM, W8_BN), (kb | k4) != 0 ? 1u : 0u);
-                        else ptx::mma_i8_ss(d_tmem, da, db, W8_IDESC, (kb | k4) != 0 ? 1u : 0u);
+                        if (F8) ptx::mma_f8_ss(d_tmem, da, db, f8_idesc(W8_BM, W8_BN), ((kb - kb0) | k4) != 0 ? 1u : 0u);
+                        else ptx::mma_i8_ss(d_tmem, da, db, W8_IDESC, ((kb - kb0) | k4) != 0 ? 1u : 0u);
                     }
                     ptx::tc_commit(empty_bar(s));
                 }
@@ -324,9 +387,9 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
         }
     } else if (warp >= 4) {
         const int q = warp - 4;                            // TMEM lane quarter this warp may read
-        int ti = 0;
+        int tile, part;
         int n_push = 0;
-        for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x, ++ti) {
+        for (int ti = 0; next_item(ti, tile, part) && !*abort_flag; ++ti) {
             const int buf = ti & 1;
             int mb_, nb_;
             w8_tile_blocks(tile, p.tiles_m, p.tiles_n, p.n_dst > 1, mb_, nb_);
@@ -348,12 +411,17 @@ gemm_w8a8_tc_kernel(const __grid_constant__ TensorMap tmA, const __grid_constant
                 }
                 const int nb = n0 + c * 32;
                 if (nb >= p.N) continue;
+                if (!F8 && p.splits > 1) {                 // warp-uniform
+                    w8_add_chunk(stage_out + q * 512, lane, row - lane, nb, r, p);
+                    continue;
+                }
                 if (!F8 && p.n_dst > 1 && nb + 32 <= p.N) {    // warp-uniform: all 32 lanes take part
                     if (p.push_tma) w8_push_chunk_tma(stage_out + q * 512, n_push++, lane, row - lane, nb, r, sa, p, dmaps);
                     else w8_push_chunk(stage_out + q * 512, lane, row - lane, nb, r, sa, p);
                 }
                 if (!row_ok) continue;
-                if (F8) f8_store_chunk(crow, nb, r, p);
+                if (F8 && p.splits > 1) f8_add_chunk(crow, nb, r, part == 0, part == p.splits - 1, p);
+                else if (F8) f8_store_chunk(crow, nb, r, p);
                 else w8_store_chunk(crow, nb, r, sa, p);
             }
         }
@@ -525,9 +593,10 @@ gemm_w8a8_tc_pair_kernel(const __grid_constant__ TensorMap tmA, const __grid_con
     }
 }
 
-bool w8a8_fast_ok(int M, int N, int K) {
-    return M >= 64 && N >= 128 && K >= 128 && (N % 16) == 0 && (K % 16) == 0;
-}
+// shapes the kernels take; w8a8_fast_ok is the documented predicate, with rows enough to fill half a tile.  Fewer rows
+// leave most of a tile empty, but the weights are what costs there.
+bool w8a8_tc_ok(int M, int N, int K) { return M >= 1 && N >= 128 && K >= 128 && (N % 16) == 0 && (K % 16) == 0; }
+bool w8a8_fast_ok(int M, int N, int K) { return M >= 64 && w8a8_tc_ok(M, N, K); }
 
 template <bool F8>
 static int launch_tc(lhb_ctx* ctx, const void* Aq, const void* Bq, W8Params p, cudaStream_t st) {
@@ -545,6 +614,7 @@ static int launch_tc(lhb_ctx* ctx, const void* Aq, const void* Bq, W8Params p, c
     }
     p.tiles_m = ceil_div(M, W8_BM); p.tiles_n = ceil_div(N, W8_BN);
     p.status = ctx->status_word;
+    p.splits = 1;
     if (p.n_dst == 0) {                                      // a plain call: one row-major [M, N] result
         p.n_dst = 1; p.dst[0] = p.C; p.ldc = N; p.col0 = 0;
     }
@@ -563,8 +633,26 @@ static int launch_tc(lhb_ctx* ctx, const void* Aq, const void* Bq, W8Params p, c
     const bool use_pair = knobs().w8a8_pair;
     // a caller that overlaps its own communication kernels keeps some SMs out of the persistent grid
     const int sms = ctx->sm_limit > 0 ? std::min(ctx->sm_count, ctx->sm_limit) : ctx->sm_count;
-    if (use_pair && M >= 256) {
-        const int tiles = ceil_div(M, 256) * p.tiles_n;
+    // Few tiles: the CTAs share K.  The parts are summed as integers in C itself (beta 0: nothing of it is read), which
+    // needs no workspace: a caller may run this beside other kernels of the context.
+    const int pair_tiles = ceil_div(M, 256) * p.tiles_n;
+    const bool pairs = use_pair && M >= 256;
+    if (!F8 && p.n_dst == 1 && p.ldc == N && p.col0 == 0 && p.beta == 0.0f && (pairs ? 4 * pair_tiles <= sms : 2 * p.tiles_m * p.tiles_n <= sms))
+        p.splits = std::max(1, std::min({sms / std::max(1, p.tiles_m * p.tiles_n), ceil_div(K, W8_BK) / 2, 16}));
+    // fp8 with few rows: the tensor core's sums lose a bit more with every doubling of K, and callers with fewer than 64 rows
+    // had sequential fp32 sums before.  Parts of 512 k, added in fp32.
+    if (F8 && M < 64) p.splits = ceil_div(K, 512);
+    if (!F8 && p.splits > 1) {
+        LHB_CUDA(cudaMemsetAsync(p.C, 0, static_cast<size_t>(M) * N * sizeof(float), st));
+        gemm_w8a8_tc_kernel<F8><<<std::min(sms, p.tiles_m * p.tiles_n * p.splits), W8_THREADS, W8_SMEM, st>>>(tmA, tmB, p, *dmaps);
+        LHB_LAUNCH_CHECK();
+        const int64_t total4 = static_cast<int64_t>(M) * N / 4;
+        LHB_CUDA(launch_pdl(w8_finish_kernel, dim3(static_cast<unsigned>(ceil_div64(total4, 256))), dim3(256), 0, st, p.C, p.a_scales, p.b_scales,
+                            p.alpha, total4, N / 4));
+        return LHB_OK;
+    }
+    if (pairs) {
+        const int tiles = pair_tiles;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2 * std::max(1, std::min(sms / 2, tiles)), 1, 1);   // at least one pair, whatever the SM limit
         cfg.blockDim = dim3(W8_THREADS, 1, 1);

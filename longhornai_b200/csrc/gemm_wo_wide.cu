@@ -555,7 +555,9 @@ bool wo_wide_ok(int fmt, int M, int N, int K, int G) {
 bool wo_wide_prefer(int fmt, int M, int N, int K, int G) {
     if (!wo_wide_ok(fmt, M, N, K, G)) return false;
     if (knobs().wo_wide_min_m > 0) return M >= knobs().wo_wide_min_m;
-    return M > 32;
+    // Two slabs of the few-row kernel still do better: 64 rows of int4 at 4096x14336 42 us against 49, at 14336x4096 40
+    // against 48; 96 rows 61 against 52.  Groups it does not take: two GEMV slabs of 16 rows are as fast as 32 rows here.
+    return M > (wo_tc_ok(fmt, M, N, K, G) ? 64 : 32);
 }
 
 template <int FMT>

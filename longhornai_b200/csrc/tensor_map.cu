@@ -115,7 +115,7 @@ const Knobs& knobs() {
         };
         v.pdl = num("LHB_PDL", 1) != 0;
         v.w4tc_min_m = std::max(1, num("LHB_W4TC_MIN_M", 9));
-        v.wo_tc_min_m = std::max(1, num("LHB_WO_TC_MIN_M", 9));
+        v.wo_tc_min_m = std::max(0, num("LHB_WO_TC_MIN_M", 0));
         v.wo_wide_min_m = std::max(0, num("LHB_WO_WIDE_MIN_M", 0));
         v.w4tc_stream_k = num("LHB_W4TC_SPLIT", 0) == 1;
         v.w4tc_ctas = std::max(0, num("LHB_W4TC_CTAS", 0));
